@@ -8,27 +8,24 @@
 // integer this kernel produces equals the GEMV's and the oracle's.  Because the
 // weight scale and the activation scale both change every 32 K, an accumulator
 // is drained from tensor memory after every K = 32 step and scaled on the CUDA
-// cores; that rescale, not the tensor pipe, bounds this kernel.
+// cores; that rescale, not the tensor pipe, bounds this kernel.  Accumulators change hands in groups (half of tensor
+// memory at a time), not run by run, and the launch overlaps the quantizer in front of it (programmatic serialization):
+// with the decode of the weight scales moved off their load, 8192 x 3072, M = 512 went from 185 to 167 us.
 //
-// One CTA = 128 weight rows x BN tokens, E + 4 warps with fixed roles:
-//   warps 0..E-1  epilogue (E = 4 per 32 token columns: 16 for BN = 128): TMEM ->
-//               registers (tcgen05.ld), f32 rescale, store
-//   next 2      unpack: packed weights (global) -> int8 tile in shared memory
+// One CTA = 128 weight rows x BN tokens (128, 64 or 32; gemm_plan), warps with fixed roles (Tile<BN>):
+//   epilogue    TMEM -> registers (tcgen05.ld), f32 rescale, store
+//   unpack      packed weights (global) -> int8 tile in shared memory
 //               (128-byte swizzle, the layout the MMA descriptor names)
-//   next 1      TMA producer: activation int8 tile + its scale tiles (and the
+//   TMA         activation int8 tile + its scale tiles (and the
 //               weight tile itself for Q8_0, whose int8 plane needs no unpacking)
-//   last        MMA issuer (one elected lane) + TMEM allocation
+//   MMA issuer  one elected lane, + TMEM allocation
+// The CTAs of a cluster may share one tile, each on its own part of K; their f32 sums meet in distributed shared memory.
 // Stages (K = 128 each) and TMEM accumulators are rings guarded by mbarriers;
 // every wait is bounded and raises the context's error word instead of
 // spinning forever.
 #include "fk_common.cuh"
 
-#ifndef FK_I2F_MASK
-#define FK_I2F_MASK 15
-#endif
-#ifndef FK_EPI_F32X2
-#define FK_EPI_F32X2 1
-#endif
+#include <math.h>
 
 #include "fk_tc.cuh"
 
@@ -50,21 +47,30 @@ __device__ __forceinline__ unsigned long long gtime_ns() {
 constexpr int BM = 128;           // weight rows per CTA (MMA M)
 constexpr int KSTAGE = 128;       // K per pipeline stage (4 MMAs of K = 32)
 constexpr int NSTAGE = 4;
-constexpr int UNPACK_WARPS = 2;
-// epilogue warps: four (one per TMEM lane quadrant) for every 32 token columns of the tile
-__host__ __device__ constexpr int epi_warps(int bn) { return bn / 32 * 4; }
-__host__ __device__ constexpr int gemm_threads(int bn) { return (epi_warps(bn) + UNPACK_WARPS + 2) * 32; }
+// Tile shapes.  BN token columns per CTA; an epilogue warp owns CW of them in one TMEM lane quadrant.
+template <int BN> struct Tile {
+    static constexpr int CW = BN >= 128 ? 32 : 16;
+    static constexpr int EPI_WARPS = BN / CW * 4;
+    static constexpr int UNPACK_WARPS = BN >= 128 ? 2 : 4;
+    static constexpr int THREADS = (EPI_WARPS + UNPACK_WARPS + 2) * 32;
+    static constexpr int BLOCKS = BN >= 64 ? 1 : 2;      // resident per SM: what shared and tensor memory are cut for
+    static constexpr int NACC = 512 / BLOCKS / BN;       // TMEM accumulators: two groups, one filled while the other is drained
+    static constexpr int GROUP = NACC / 2;               // runs that share one hand-over (a commit, a wait, a release)
+};
+constexpr int MAX_SPLIT = 8;      // CTAs of a cluster that share one tile, each on its own part of K
 
 struct GemmArgs {
     const uint8_t* w;         // matrix 0 of the weight handle
     size_t mat_stride;
     size_t plane_off[4];
     size_t plane_stride[4];
-    int kind, rows, cols;
+    int rows, cols;
     int mat;                  // dense: the matrix; grouped: ignored
     const int* tile_expert;   // grouped: expert of each token tile (nullptr = dense)
     const int* n_tiles_dev;   // grouped: number of live token tiles (nullptr = all of gridDim.y)
-    const int* out_row;       // padded token row -> output row, -1 = padding
+    const int* out_row;       // padded token row -> output row, -1 = padding (nullptr = dense: row t is token t, padding from m on)
+    int m;
+    int split;                // CTAs per tile along K (the cluster's size in z)
     float* out;
     int32_t* isums;           // test hook: the raw accumulators, [token][rows][cols / run] (nullptr = off)
     int* err;
@@ -78,71 +84,83 @@ template <int BN> struct Smem {
     static constexpr int STAGE = A_BYTES + B_BYTES + 2 * DX_BYTES;
     static constexpr int BARS = NSTAGE * STAGE;          // barrier block
     static constexpr int TOTAL = BARS + 256 + 1024;      // + alignment slack
-    static constexpr int NACC = 512 / BN;                // TMEM accumulator ring
+    static_assert(BM * BN * 4 <= BARS, "the partial sums of a split tile reuse the stages");
 };
 
-// Weight scale of row `row`, run `kb`; Q4_K also the min scale.  Q6_K rows are
-// (weight row, half-run) pairs, see the unpack warps.
-struct WScale { float dw, mw; };
+// The weight scales of one tile row for one stage (runs kb0 .. kb0 + 3): as loaded, and decoded.  The load is issued a
+// stage ahead and nothing touches its registers until that stage begins -- decoding at the load, as this once did, made
+// every warp wait out a global-memory latency per stage (2000 of 7600 cycles of a 128-token tile).
+template <int KIND> struct RawScale {
+    uint4 hd;        // Q4_K: d, dmin and the packed scales
+    uint2 sc;        // Q8_0: four f16; Q6_K: eight int8 (two per run); MXFP4: four exponents in x
+    uint16_t d;      // Q6_K
+};
+struct StageScale { uint32_t sc, mn; float d, dmin; uint2 raw; };
 
 template <int KIND>
-__device__ __forceinline__ void load_wscales(const GemmArgs& a, const uint8_t* wb, int row, bool row_ok, int kb0, int nkb, WScale* ws) {
-    // scales of runs kb0 .. kb0+3 of this thread's row
-#pragma unroll
-    for (int j = 0; j < 4; j++) ws[j] = {0.0f, 0.0f};
-    if (!row_ok) return;
+__device__ __forceinline__ RawScale<KIND> load_wscales(const GemmArgs& a, const uint8_t* wb, int row, bool row_ok, int kb0) {
+    RawScale<KIND> v;
+    v.hd = make_uint4(0, 0, 0, 0);
+    v.sc = make_uint2(0, 0);
+    v.d = 0;
+    if (!row_ok) return v;
     if (KIND == FK_Q4_K) {
-        const int sb = kb0 >> 3;
-        const uint4 hd = ldg16(wb + ((size_t)row * (a.cols >> 8) + sb) * 144);
-        const float d = fk_h2f((uint16_t)(hd.x & 0xFFFF)), dmin = fk_h2f((uint16_t)(hd.x >> 16));
-        const uint32_t s[3] = {hd.y, hd.z, hd.w};
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int q = (kb0 & 7) + j;  // sub-block 0..7
-            uint32_t sc, m;
-            if (q < 4) {
-                sc = (s[0] >> (8 * q)) & 63;
-                m = (s[1] >> (8 * q)) & 63;
-            } else {
-                const uint32_t b = (s[2] >> (8 * (q - 4))) & 0xFF;
-                sc = (b & 0x0F) | ((((s[0] >> (8 * (q - 4))) & 0xFF) >> 6) << 4);
-                m = (b >> 4) | ((((s[1] >> (8 * (q - 4))) & 0xFF) >> 6) << 4);
-            }
-            if (kb0 + j < nkb) ws[j] = {d * (float)sc, dmin * (float)m};
-        }
+        v.hd = ldg16(wb + ((size_t)row * (a.cols >> 8) + (kb0 >> 3)) * 144);
     } else if (KIND == FK_Q8_0) {
-        const uint16_t* dp = (const uint16_t*)(wb + a.plane_off[1] + (size_t)row * a.plane_stride[1]);
-#pragma unroll
-        for (int j = 0; j < 4; j++)
-            if (kb0 + j < nkb) ws[j].dw = fk_h2f(__ldg(dp + kb0 + j));
+        v.sc = __ldg((const uint2*)(wb + a.plane_off[1] + (size_t)row * a.plane_stride[1] + 2 * kb0));   // rows are padded to 16 bytes
     } else if (KIND == FK_MXFP4) {
-        const uint8_t* ep = wb + a.plane_off[1] + (size_t)row * a.plane_stride[1];
-#pragma unroll
-        for (int j = 0; j < 4; j++)
-            if (kb0 + j < nkb) ws[j].dw = e8m0_half(__ldg(ep + kb0 + j));
-    } else {  // FK_Q6_K: `row` = 2 * weight row + half; its scale of run kb is sc[2 * kb + half]
-        const int wrow = row >> 1, half = row & 1;
-        const int sb = kb0 >> 3;
-        const float d = fk_h2f(__ldg((const uint16_t*)(wb + a.plane_off[3] + (size_t)wrow * a.plane_stride[3]) + sb));
-        const int8_t* sc = (const int8_t*)(wb + a.plane_off[2] + (size_t)wrow * a.plane_stride[2]) + 2 * kb0 + half;
-#pragma unroll
-        for (int j = 0; j < 4; j++)
-            if (kb0 + j < nkb) ws[j].dw = d * (float)__ldg(sc + 2 * j);
+        v.sc.x = __ldg((const uint32_t*)(wb + a.plane_off[1] + (size_t)row * a.plane_stride[1] + kb0));
+    } else {  // FK_Q6_K: `row` = 2 * weight row + half
+        const int wrow = row >> 1;
+        v.d = __ldg((const uint16_t*)(wb + a.plane_off[3] + (size_t)wrow * a.plane_stride[3]) + (kb0 >> 3));
+        v.sc = __ldg((const uint2*)(wb + a.plane_off[2] + (size_t)wrow * a.plane_stride[2] + 2 * kb0));
+    }
+    return v;
+}
+template <int KIND>
+__device__ __forceinline__ StageScale stage_scales(const RawScale<KIND>& v, int kb0) {
+    StageScale t{};
+    if (KIND == FK_Q4_K) {
+        t.d = fk_h2f((uint16_t)(v.hd.x & 0xFFFF));
+        t.dmin = fk_h2f((uint16_t)(v.hd.x >> 16));
+        // 6-bit scales and mins of sub-blocks 0..3 or 4..7, one per byte
+        t.sc = (kb0 & 4) ? (v.hd.w & 0x0F0F0F0Fu) | ((v.hd.y >> 2) & 0x30303030u) : v.hd.y & 0x3F3F3F3Fu;
+        t.mn = (kb0 & 4) ? ((v.hd.w >> 4) & 0x0F0F0F0Fu) | ((v.hd.z >> 2) & 0x30303030u) : v.hd.z & 0x3F3F3F3Fu;
+    } else {
+        if (KIND == FK_Q6_K) t.d = fk_h2f(v.d);
+        t.raw = v.sc;
+    }
+    return t;
+}
+// Scale (and, Q4_K, min scale) of run kb0 + j.
+template <int KIND>
+__device__ __forceinline__ void run_scale(const StageScale& t, int j, int row, float* dw, float* mw) {
+    *mw = 0.0f;
+    if (KIND == FK_Q4_K) {
+        *dw = t.d * (float)((t.sc >> (8 * j)) & 0xFFu);
+        *mw = t.dmin * (float)((t.mn >> (8 * j)) & 0xFFu);
+    } else if (KIND == FK_Q8_0) {
+        *dw = fk_h2f((uint16_t)((j < 2 ? t.raw.x : t.raw.y) >> (16 * (j & 1))));
+    } else if (KIND == FK_MXFP4) {
+        *dw = e8m0_half((t.raw.x >> (8 * j)) & 0xFFu);
+    } else {
+        *dw = t.d * (float)(int8_t)((j < 2 ? t.raw.x : t.raw.y) >> (16 * (j & 1) + 8 * (row & 1)));
     }
 }
 
-// Packed bytes of one weight row for stage `st` (K range [128 st, 128 st + 128)),
-// as loaded (nothing decoded yet, so the loads of the next stage can be in
-// flight while this stage is written).
-template <int KIND> struct RawRow { uint4 q[KIND == FK_Q6_K ? 6 : 4]; };
+// Packed bytes of one TILE row for stage `st` (K range [128 st, 128 st + 128)), as loaded (nothing decoded yet, so the
+// loads of the next stages can be in flight while this stage is written).  Q6_K: tile row r is half r & 1 of weight row
+// r >> 1, and takes the 16 bytes of every plane piece that hold its half.
+template <int KIND> struct RawRow { uint4 q[KIND == FK_Q6_K ? 3 : 4]; };
 
 template <int KIND>
-__device__ __forceinline__ void load_raw(const GemmArgs& a, const uint8_t* wb, int wrow, bool ok, int st, RawRow<KIND>& raw) {
-    constexpr int N = KIND == FK_Q6_K ? 6 : 4;
+__device__ __forceinline__ void load_raw(const GemmArgs& a, const uint8_t* wb, int wrow0, int r, int st, bool live, RawRow<KIND>& raw) {
+    constexpr int N = KIND == FK_Q6_K ? 3 : 4;
 #pragma unroll
     for (int i = 0; i < N; i++) raw.q[i] = make_uint4(0, 0, 0, 0);
     const int k0 = st * KSTAGE;
-    if (!ok || k0 >= a.cols || KIND == FK_Q8_0) return;
+    const int wrow = wrow0 + (KIND == FK_Q6_K ? r >> 1 : r);
+    if (!live || wrow >= a.rows || k0 >= a.cols || KIND == FK_Q8_0) return;
     if (KIND == FK_Q4_K) {
         // 128 weights = 64 quant bytes: two groups of 32 bytes
         const uint8_t* p = wb + ((size_t)wrow * (a.cols >> 8) + (k0 >> 8)) * 144 + 16 + ((k0 >> 7) & 1) * 64;
@@ -153,28 +171,19 @@ __device__ __forceinline__ void load_raw(const GemmArgs& a, const uint8_t* wb, i
 #pragma unroll
         for (int b = 0; b < 4; b++)
             if (k0 + 32 * b < a.cols) raw.q[b] = ldg16(p + 16 * b);
-    } else {  // FK_Q6_K: 64 ql bytes + 32 qh bytes of this half super-block
-        const int sb = k0 >> 8, hf = (k0 >> 7) & 1;
-        const uint8_t* ql = wb + a.plane_off[0] + (size_t)wrow * (a.cols >> 1) + (size_t)sb * 128 + 64 * hf;
-        const uint8_t* qh = wb + a.plane_off[1] + (size_t)wrow * (a.cols >> 2) + (size_t)sb * 64 + 32 * hf;
-#pragma unroll
-        for (int i = 0; i < 4; i++) raw.q[i] = ldg16(ql + 16 * i);
-        raw.q[4] = ldg16(qh);
-        raw.q[5] = ldg16(qh + 16);
+    } else {  // FK_Q6_K: of the 64 ql bytes and 32 qh bytes of this half super-block, those of bytes 16 h .. 16 h + 15 of every 32
+        const int sb = k0 >> 8, hf = (k0 >> 7) & 1, h = 16 * (r & 1);
+        const uint8_t* ql = wb + a.plane_off[0] + (size_t)wrow * (a.cols >> 1) + (size_t)sb * 128 + 64 * hf + h;
+        const uint8_t* qh = wb + a.plane_off[1] + (size_t)wrow * (a.cols >> 2) + (size_t)sb * 64 + 32 * hf + h;
+        raw.q[0] = ldg16(ql);
+        raw.q[1] = ldg16(ql + 32);
+        raw.q[2] = ldg16(qh);
     }
 }
 
-__device__ __forceinline__ void store_tile_row(uint8_t* a_tile, int r, const uint4* o) {
-    uint8_t* dst = a_tile + r * 128;
-#pragma unroll
-    for (int c = 0; c < 8; c++) *(uint4*)(dst + ((c ^ (r & 7)) << 4)) = o[c];
-}
-
-// Decode one weight row's 128 weights of a stage to int8 and write them as tile
-// row(s), eight 16-byte chunks each at their swizzled places.  Q4_K, MXFP4:
-// tile row `r`.  Q6_K: tile rows 2 r' and 2 r' + 1 (r = 2 r'), the codes minus
-// 32 with the 16 weights of the OTHER half of every run of 32 zeroed, so that
-// one K = 32 MMA yields the exact dot of a 16-weight scale group.
+// Decode one tile row's 128 weights of a stage to int8 and write them, eight 16-byte chunks each at their swizzled
+// places.  Q6_K: the codes minus 32 with the 16 weights of the OTHER half of every run of 32 zeroed, so that one K = 32
+// MMA yields the exact dot of a 16-weight scale group.
 template <int KIND>
 __device__ __forceinline__ void store_raw(const RawRow<KIND>& raw, int r, uint8_t* a_tile) {
     uint4 o[8];
@@ -188,7 +197,6 @@ __device__ __forceinline__ void store_raw(const RawRow<KIND>& raw, int r, uint8_
             o[4 * g + 2] = make_uint4((q0.x >> 4) & 0x0F0F0F0Fu, (q0.y >> 4) & 0x0F0F0F0Fu, (q0.z >> 4) & 0x0F0F0F0Fu, (q0.w >> 4) & 0x0F0F0F0Fu);
             o[4 * g + 3] = make_uint4((q1.x >> 4) & 0x0F0F0F0Fu, (q1.y >> 4) & 0x0F0F0F0Fu, (q1.z >> 4) & 0x0F0F0F0Fu, (q1.w >> 4) & 0x0F0F0F0Fu);
         }
-        store_tile_row(a_tile, r, o);
     } else if (KIND == FK_MXFP4) {
         // bytes come out as (elem j, elem j+16) pairs, the order the activation
         // plane of this kind is stored in; an absent block (past the last column) is zeros
@@ -198,46 +206,60 @@ __device__ __forceinline__ void store_raw(const RawRow<KIND>& raw, int r, uint8_
             o[2 * b] = make_uint4(e2m1x2_4(q.x), e2m1x2_4(q.x >> 16), e2m1x2_4(q.y), e2m1x2_4(q.y >> 16));
             o[2 * b + 1] = make_uint4(e2m1x2_4(q.z), e2m1x2_4(q.z >> 16), e2m1x2_4(q.w), e2m1x2_4(q.w >> 16));
         }
-        store_tile_row(a_tile, r, o);
     } else if (KIND == FK_Q6_K) {
-        const uint32_t hh[8] = {raw.q[4].x, raw.q[4].y, raw.q[4].z, raw.q[4].w, raw.q[5].x, raw.q[5].y, raw.q[5].z, raw.q[5].w};
-        uint4 o1[8];
-        // element e = 32 * qd + l (qd = 0..3, l = 0..31): ql byte (l + 32 * (qd & 1)),
-        // nibble (qd >> 1), qh byte l bits [2 qd, 2 qd + 2)
+        // element e = 32 * qd + 16 * half + l (qd = 0..3): nibble (qd >> 1) of ql piece (qd & 1), qh bits [2 qd, 2 qd + 2)
+        const uint32_t hh[4] = {raw.q[2].x, raw.q[2].y, raw.q[2].z, raw.q[2].w};
+        const bool odd = r & 1;
 #pragma unroll
         for (int qd = 0; qd < 4; qd++) {
-            const uint4 l0 = raw.q[2 * (qd & 1)], l1 = raw.q[2 * (qd & 1) + 1];
-            const uint32_t ll[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
-            uint32_t v[8];
+            const uint4 l0 = raw.q[qd & 1];
+            const uint32_t ll[4] = {l0.x, l0.y, l0.z, l0.w};
+            uint32_t v[4];
 #pragma unroll
-            for (int i = 0; i < 8; i++) {
+            for (int i = 0; i < 4; i++) {
                 const uint32_t nib = (qd >> 1) ? ((ll[i] >> 4) & 0x0F0F0F0Fu) : (ll[i] & 0x0F0F0F0Fu);
-                const uint32_t c6 = nib | (((hh[i] >> (2 * qd)) & 0x03030303u) << 4);
-                v[i] = __vsub4(c6, 0x20202020u);
+                v[i] = __vsub4(nib | (((hh[i] >> (2 * qd)) & 0x03030303u) << 4), 0x20202020u);
             }
-            o[2 * qd] = make_uint4(v[0], v[1], v[2], v[3]);       // half 0 keeps the first 16 of the run
-            o[2 * qd + 1] = make_uint4(0, 0, 0, 0);
-            o1[2 * qd] = make_uint4(0, 0, 0, 0);
-            o1[2 * qd + 1] = make_uint4(v[4], v[5], v[6], v[7]);  // half 1 the last 16
+            const uint4 val = make_uint4(v[0], v[1], v[2], v[3]), zero = make_uint4(0, 0, 0, 0);
+            o[2 * qd] = odd ? zero : val;
+            o[2 * qd + 1] = odd ? val : zero;
         }
-        store_tile_row(a_tile, r, o);
-        store_tile_row(a_tile, r + 1, o1);
     }
+    uint8_t* dst = a_tile + r * 128;
+#pragma unroll
+    for (int c = 0; c < 8; c++) *(uint4*)(dst + ((c ^ (r & 7)) << 4)) = o[c];
+}
+
+__device__ __forceinline__ float ld_cluster_f32(uint32_t addr, int rank) {
+    uint32_t remote;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote));
+    return v;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 template <int KIND, int BN, bool DUMP>
-__global__ void __launch_bounds__(gemm_threads(BN), 1)
+__global__ void __launch_bounds__(Tile<BN>::THREADS, Tile<BN>::BLOCKS)
 gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_dx,
             const __grid_constant__ CUtensorMap map_sx, const __grid_constant__ CUtensorMap map_w) {
     using S = Smem<BN>;
-    constexpr int EPI_WARPS = epi_warps(BN);
+    using T = Tile<BN>;
+    constexpr int EPI_WARPS = T::EPI_WARPS, UNPACK_WARPS = T::UNPACK_WARPS, NACC = T::NACC, G = T::GROUP, CW = T::CW, HC = CW / 2;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const uint32_t sbase = smem_u32(smem);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
+    // Only weights (constants) may be read before the quantizer in front of this launch has finished; the grouped form's
+    // tile list is the work of the kernels before that.
     const int ttile = blockIdx.y;
-    if (a.n_tiles_dev && ttile >= *a.n_tiles_dev) return;
+    if (a.n_tiles_dev) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        if (ttile >= *a.n_tiles_dev) return;       // every CTA of the cluster alike
+    }
     const int mat = a.tile_expert ? a.tile_expert[ttile] : a.mat;
     const uint8_t* wb = a.w + (size_t)mat * a.mat_stride;
     // Q6_K tile rows are (weight row, half) pairs: 64 weight rows per CTA
@@ -245,16 +267,20 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap map_q, const _
     const int wrow0 = blockIdx.x * WROWS;
     const int tok0 = ttile * BN;
     const int nkb = a.cols >> 5;
-    const int nst = (nkb + 3) >> 2;
+    const int nst_all = (nkb + 3) >> 2;
+    // this CTA's stages: [st0, st0 + nst) of the row, runs kb_lo .. kb_lo + nkl - 1
+    const int rank = blockIdx.z, split = a.split;
+    const int st0 = (int)((long long)nst_all * rank / split), nst = (int)((long long)nst_all * (rank + 1) / split) - st0;
+    const int kb_lo = 4 * st0, nkl = min(nkb - kb_lo, 4 * nst);
 
-    // barriers: full_b[NSTAGE], full_a[NSTAGE], empty[NSTAGE], acc_full[NACC], acc_empty[NACC], then the TMEM base word
+    // barriers: full_b[NSTAGE], full_a[NSTAGE], empty[NSTAGE], acc_full[2], acc_empty[2], then the TMEM base word
     const uint32_t bar0 = sbase + S::BARS;
     auto full_b = [&](int s) { return bar0 + 8u * s; };
     auto full_a = [&](int s) { return bar0 + 8u * (NSTAGE + s); };
     auto empty = [&](int s) { return bar0 + 8u * (2 * NSTAGE + s); };
     auto acc_full = [&](int b) { return bar0 + 8u * (3 * NSTAGE + b); };
-    auto acc_empty = [&](int b) { return bar0 + 8u * (3 * NSTAGE + S::NACC + b); };
-    uint32_t* tmem_word = (uint32_t*)(smem + S::BARS + 8 * (3 * NSTAGE + 2 * S::NACC));
+    auto acc_empty = [&](int b) { return bar0 + 8u * (3 * NSTAGE + 2 + b); };
+    uint32_t* tmem_word = (uint32_t*)(smem + S::BARS + 8 * (3 * NSTAGE + 4));
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < NSTAGE; s++) {
@@ -262,14 +288,14 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap map_q, const _
             mbar_init(full_a(s), UNPACK_WARPS);
             mbar_init(empty(s), 1 + EPI_WARPS);
         }
-        for (int b = 0; b < S::NACC; b++) {
+        for (int b = 0; b < 2; b++) {
             mbar_init(acc_full(b), 1);
             mbar_init(acc_empty(b), EPI_WARPS);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == EPI_WARPS + UNPACK_WARPS + 1) {  // the MMA warp owns tensor memory
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_word)), "r"(512) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_word)), "r"(NACC * BN) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     tc_fence_before();
@@ -277,40 +303,41 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap map_q, const _
     tc_fence_after();
     const uint32_t tmem_base = *tmem_word;
 
+    auto out_row_of = [&](int t) { return a.out_row ? a.out_row[t] : (t < a.m ? t : -1); };
     if (warp < EPI_WARPS) {
         // ------------------------------------------------------------ epilogue
         const int quad = warp & 3, chalf = warp >> 2;
         const int r = quad * 32 + lane;                // tile row = TMEM lane
         const int row = KIND == FK_Q6_K ? 2 * wrow0 + r : wrow0 + r;   // scale row id (pair id for Q6_K)
         const bool row_ok = (KIND == FK_Q6_K ? (wrow0 + (r >> 1)) : (wrow0 + r)) < a.rows;
-        constexpr int CW = 32;                         // token columns this warp owns
-        float acc[CW];
+        const int orow = KIND == FK_Q6_K ? wrow0 + (r >> 1) : wrow0 + r;
+        const bool writer = row_ok && (KIND != FK_Q6_K || !(r & 1));
+        float acc[CW];                                 // CW token columns of one row
 #pragma unroll
         for (int i = 0; i < CW; i++) acc[i] = 0.0f;
         const uint32_t taddr0 = tmem_base + ((uint32_t)(quad * 32) << 16) + chalf * CW;
-        WScale ws[4], ws_next[4];
-        load_wscales<KIND>(a, wb, row, row_ok, 0, nkb, ws_next);
-        // TMEM reads are double-buffered in halves of 16 columns: while one half is
+        RawScale<KIND> ws_next = load_wscales<KIND>(a, wb, row, row_ok, kb_lo);
+        if (!a.n_tiles_dev) asm volatile("griddepcontrol.wait;" ::: "memory");
+        // TMEM reads are double-buffered in halves of HC columns: while one half is
         // scaled the next one (or the next run's first) is already in flight, so a warp's
         // chain per run is its arithmetic, not the accumulator hand-off latency.
-        uint32_t v[2][16];
-        auto issue = [&](int kb, int c, uint32_t* dst) {
-            const int buf = kb % S::NACC;
-            if (c == 0) {
-                mbar_wait(acc_full(buf), (kb / S::NACC) & 1, a.err, 11);
+        uint32_t v[2][HC];
+        auto issue = [&](int kb, int c, uint32_t* dst) {   // kb counts from this CTA's first run
+            if (c == 0 && kb % G == 0) {
+                mbar_wait(acc_full((kb / G) & 1), (kb / NACC) & 1, a.err, 11);
                 tc_fence_after();
                 GTR(1, kb, warp == 0 && lane == 0);
             }
-            tc_ld16(taddr0 + buf * BN + c * 16, dst);
+            if (HC == 16) tc_ld16(taddr0 + (kb % NACC) * BN + c * HC, dst);
+            else tc_ld8(taddr0 + (kb % NACC) * BN + c * HC, dst);
         };
         issue(0, 0, v[0]);
         tc_wait_ld();
-        tc_ld_fence<16>(v[0]);
+        tc_ld_fence<HC>(v[0]);
         for (int st = 0; st < nst; st++) {
             const int s = st % NSTAGE;
-#pragma unroll
-            for (int j = 0; j < 4; j++) ws[j] = ws_next[j];
-            if (st + 1 < nst) load_wscales<KIND>(a, wb, row, row_ok, 4 * (st + 1), nkb, ws_next);
+            const StageScale ws = stage_scales<KIND>(ws_next, kb_lo + 4 * st);
+            if (st + 1 < nst) ws_next = load_wscales<KIND>(a, wb, row, row_ok, kb_lo + 4 * (st + 1));
             mbar_wait(full_b(s), (st / NSTAGE) & 1, a.err, 10);   // the scale tiles of this stage have landed
             // the stage's scale tiles: dx [4][BN] then (Q4_K) sx [4][BN], as shared-space addresses
             const uint32_t sdx_s = sbase + s * S::STAGE + S::A_BYTES + S::B_BYTES;
@@ -318,27 +345,27 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap map_q, const _
 #pragma unroll 1
             for (int j = 0; j < 4; j++) {
                 const int kb = 4 * st + j;
-                if (kb >= nkb) break;
-                const float dw = j == 0 ? ws[0].dw : (j == 1 ? ws[1].dw : (j == 2 ? ws[2].dw : ws[3].dw));
-                const float mw = j == 0 ? ws[0].mw : (j == 1 ? ws[1].mw : (j == 2 ? ws[2].mw : ws[3].mw));
+                if (kb >= nkl) break;
+                float dw, mw;
+                run_scale<KIND>(ws, j, row, &dw, &mw);
 #pragma unroll
                 for (int c = 0; c < 2; c++) {
                     uint32_t* cur = v[c];
                     uint32_t* nxt = v[c ^ 1];
                     const int kb_n = c == 0 ? kb : kb + 1, c_n = c ^ 1;
-                    if (kb_n < nkb) issue(kb_n, c_n, nxt);
-                    const uint32_t dxs = sdx_s + (uint32_t)(j * BN + chalf * CW + c * 16) * 4u;
+                    if (kb_n < nkl) issue(kb_n, c_n, nxt);
+                    const uint32_t dxs = sdx_s + (uint32_t)(j * BN + chalf * CW + c * HC) * 4u;
                     if (DUMP && row_ok) {
                         // the exact integers of this run, before any scale touches them
                         const int orow_d = KIND == FK_Q6_K ? wrow0 + (r >> 1) : wrow0 + r;
-                        const int nruns = KIND == FK_Q6_K ? a.cols >> 4 : nkb, run = KIND == FK_Q6_K ? 2 * kb + (r & 1) : kb;
-                        for (int i = 0; i < 16; i++) {
-                            const int dst = a.out_row[tok0 + chalf * CW + c * 16 + i];
+                        const int nruns = KIND == FK_Q6_K ? a.cols >> 4 : nkb, run = KIND == FK_Q6_K ? 2 * (kb_lo + kb) + (r & 1) : kb_lo + kb;
+                        for (int i = 0; i < HC; i++) {
+                            const int dst = out_row_of(tok0 + chalf * CW + c * HC + i);
                             if (dst >= 0) a.isums[((size_t)dst * a.rows + orow_d) * nruns + run] = (int32_t)cur[i];
                         }
                     }
 #pragma unroll
-                    for (int i = 0; i < 16; i += 4) {
+                    for (int i = 0; i < HC; i += 4) {
                         const float4 dx = lds128(dxs + 4u * i);
                         const float dxa[4] = {dx.x, dx.y, dx.z, dx.w};
                         float sxa[4] = {0.0f, 0.0f, 0.0f, 0.0f};
@@ -346,50 +373,25 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap map_q, const _
                             const float4 sx = lds128(dxs + 16u * BN + 4u * i);
                             sxa[0] = sx.x; sxa[1] = sx.y; sxa[2] = sx.z; sxa[3] = sx.w;
                         }
-#if FK_EPI_F32X2
-                        // two columns per instruction on the packed f32x2 path; int32 -> f32 (exact, |C| < 2^22)
-                        // either on the conversion unit (bit of FK_I2F_MASK set: one issue slot, a quarter of
-                        // the rate) or by the magic-number add on the integer and FP32 pipes (two slots)
+                        // two columns per instruction on the packed f32x2 path; int32 -> f32 (exact, |C| < 2^22) on the
+                        // conversion unit: one issue slot, where the magic-number add takes two on the integer and FP32 pipes
 #pragma unroll
                         for (int e = 0; e < 4; e += 2) {
-                            constexpr int M2 = FK_I2F_MASK;
-                            float2 f2;
-                            if (((M2 >> e) & 3) == 3) {
-                                f2 = make_float2((float)(int)cur[i + e], (float)(int)cur[i + e + 1]);
-                            } else if (((M2 >> e) & 3) == 0) {
-                                f2 = __fadd2_rn(make_float2(__int_as_float((int)cur[i + e] + 0x4B400000), __int_as_float((int)cur[i + e + 1] + 0x4B400000)),
-                                                make_float2(-12582912.0f, -12582912.0f));
-                            } else {
-                                f2.x = ((M2 >> e) & 1) ? (float)(int)cur[i + e] : __int_as_float((int)cur[i + e] + 0x4B400000) - 12582912.0f;
-                                f2.y = ((M2 >> e) & 2) ? (float)(int)cur[i + e + 1] : __int_as_float((int)cur[i + e + 1] + 0x4B400000) - 12582912.0f;
-                            }
+                            const float2 f2 = make_float2((float)(int)cur[i + e], (float)(int)cur[i + e + 1]);
                             const float2 s2 = __fmul2_rn(make_float2(dw, dw), make_float2(dxa[e], dxa[e + 1]));
-                            float2 t2 = __ffma2_rn(s2, f2, make_float2(acc[c * 16 + i + e], acc[c * 16 + i + e + 1]));
+                            float2 t2 = __ffma2_rn(s2, f2, make_float2(acc[c * HC + i + e], acc[c * HC + i + e + 1]));
                             if (KIND == FK_Q4_K) t2 = __ffma2_rn(make_float2(-mw, -mw), make_float2(sxa[e], sxa[e + 1]), t2);
-                            acc[c * 16 + i + e] = t2.x;
-                            acc[c * 16 + i + e + 1] = t2.y;
+                            acc[c * HC + i + e] = t2.x;
+                            acc[c * HC + i + e + 1] = t2.y;
                         }
-#else
-#pragma unroll
-                        for (int e = 0; e < 4; e++) {
-                            // exact int32 -> f32 for |C| < 2^22: by the magic-number add on the integer and
-                            // FP32 pipes, or (elements whose bit of FK_I2F_MASK is set) by the conversion unit,
-                            // which costs one issue slot instead of two but runs at a quarter of the rate
-                            const float f = ((FK_I2F_MASK >> e) & 1) ? (float)(int)cur[i + e]
-                                                                     : __int_as_float((int)cur[i + e] + 0x4B400000) - 12582912.0f;
-                            float t = fmaf(dw * dxa[e], f, acc[c * 16 + i + e]);
-                            if (KIND == FK_Q4_K) t = fmaf(-mw, sxa[e], t);
-                            acc[c * 16 + i + e] = t;
-                        }
-#endif
                     }
                     tc_wait_ld();
-                    tc_ld_fence<16>(nxt);
+                    tc_ld_fence<HC>(nxt);
                     GTR(2, kb, warp == 0 && lane == 0 && c == 1);
-                    if (kb_n < nkb && c_n == 1) {   // both halves of that accumulator are in registers: hand it back
+                    if (kb_n < nkl && c_n == 1 && (kb_n % G == G - 1 || kb_n == nkl - 1)) {   // the group's last half is in registers: hand it back
                         tc_fence_before();
                         __syncwarp();
-                        if (lane == 0) mbar_arrive(acc_empty(kb_n % S::NACC));
+                        if (lane == 0) mbar_arrive(acc_empty((kb_n / G) & 1));
                     }
                 }
             }
@@ -397,44 +399,54 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap map_q, const _
             __syncwarp();
             if (lane == 0) mbar_arrive(empty(s));
         }
-        // ---- store: out[out_row[token]][weight row]
-        const int orow = KIND == FK_Q6_K ? wrow0 + (r >> 1) : wrow0 + r;
-        const bool writer = row_ok && (KIND != FK_Q6_K || !(r & 1));
+        if (split == 1) {
+            // ---- store: out[out_row[token]][weight row]
 #pragma unroll 4
-        for (int i = 0; i < CW; i++) {
-            float v0 = acc[i];
-            if (KIND == FK_Q6_K) v0 += __shfl_xor_sync(0xffffffffu, v0, 1);   // the two halves of a weight row sit in neighbouring lanes
-            const int dst = a.out_row[tok0 + chalf * CW + i];
-            if (writer && dst >= 0) a.out[(size_t)dst * a.rows + orow] = v0;
+            for (int i = 0; i < CW; i++) {
+                float v0 = acc[i];
+                if (KIND == FK_Q6_K) v0 += __shfl_xor_sync(0xffffffffu, v0, 1);   // the two halves of a weight row sit in neighbouring lanes
+                const int dst = out_row_of(tok0 + chalf * CW + i);
+                if (writer && dst >= 0) a.out[(size_t)dst * a.rows + orow] = v0;
+            }
+        } else {
+            // every epilogue warp is past its last read of the stages' scale tiles, and the last accumulator was read, so no
+            // copy or MMA touches the stages any more: they hold this part's sums, [token column][tile row]
+            asm volatile("bar.sync 1, %0;" ::"r"(EPI_WARPS * 32) : "memory");
+            float* part = (float*)smem;
+#pragma unroll
+            for (int i = 0; i < CW; i++) part[(chalf * CW + i) * BM + r] = acc[i];
         }
     } else if (warp < EPI_WARPS + UNPACK_WARPS) {
         // ------------------------------------------------- weight unpack warps
         if (KIND != FK_Q8_0) {
-            // 64 threads: Q6_K one weight row (two tile rows) each, the others two rows each
-            constexpr int NR = KIND == FK_Q6_K ? 1 : 2;
+            // a thread owns NR tile rows; the loads of the next DEPTH stages are in flight while a stage is written
+            constexpr int NR = BM / (32 * UNPACK_WARPS), DEPTH = NR == 1 ? 2 : 1;
             const int t = (warp - EPI_WARPS) * 32 + lane;
-            RawRow<KIND> cur[NR], nxt[NR];
+            RawRow<KIND> raw[DEPTH + 1][NR];
 #pragma unroll
-            for (int i = 0; i < NR; i++) load_raw<KIND>(a, wb, wrow0 + t + 64 * i, wrow0 + t + 64 * i < a.rows, 0, cur[i]);
+            for (int p = 0; p < DEPTH; p++)
+#pragma unroll
+                for (int i = 0; i < NR; i++) load_raw<KIND>(a, wb, wrow0, t + 32 * UNPACK_WARPS * i, st0 + p, p < nst, raw[p][i]);
             for (int st = 0; st < nst; st++) {
                 const int s = st % NSTAGE;
-                if (st + 1 < nst) {
 #pragma unroll
-                    for (int i = 0; i < NR; i++) load_raw<KIND>(a, wb, wrow0 + t + 64 * i, wrow0 + t + 64 * i < a.rows, st + 1, nxt[i]);
-                }
+                for (int i = 0; i < NR; i++) load_raw<KIND>(a, wb, wrow0, t + 32 * UNPACK_WARPS * i, st0 + st + DEPTH, st + DEPTH < nst, raw[DEPTH][i]);
                 if (st >= NSTAGE) mbar_wait(empty(s), ((st / NSTAGE) - 1) & 1, a.err, 20);
 #pragma unroll
-                for (int i = 0; i < NR; i++) store_raw<KIND>(cur[i], KIND == FK_Q6_K ? 2 * t : t + 64 * i, smem + s * S::STAGE);
+                for (int i = 0; i < NR; i++) store_raw<KIND>(raw[0][i], t + 32 * UNPACK_WARPS * i, smem + s * S::STAGE);
                 fence_proxy_async();   // generic-proxy writes -> visible to the tensor core's reads
                 __syncwarp();
                 if (lane == 0) mbar_arrive(full_a(s));
                 GTR(3, st, warp == EPI_WARPS && lane == 0);
 #pragma unroll
-                for (int i = 0; i < NR; i++) cur[i] = nxt[i];
+                for (int p = 0; p < DEPTH; p++)
+#pragma unroll
+                    for (int i = 0; i < NR; i++) raw[p][i] = raw[p + 1][i];
             }
         }
     } else if (warp == EPI_WARPS + UNPACK_WARPS) {
         // --------------------------------------------------------- TMA producer
+        if (!a.n_tiles_dev) asm volatile("griddepcontrol.wait;" ::: "memory");
         if (lane == 0) {
             constexpr uint32_t TX = S::B_BYTES + S::DX_BYTES + (KIND == FK_Q4_K ? S::DX_BYTES : 0) + (KIND == FK_Q8_0 ? S::A_BYTES : 0);
             for (int st = 0; st < nst; st++) {
@@ -442,10 +454,10 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap map_q, const _
                 if (st >= NSTAGE) mbar_wait(empty(s), ((st / NSTAGE) - 1) & 1, a.err, 30);
                 const uint32_t sa = sbase + s * S::STAGE;
                 mbar_expect_tx(full_b(s), TX);
-                tma_load_2d(sa + S::A_BYTES, &map_q, st * KSTAGE, tok0, full_b(s));
-                tma_load_2d(sa + S::A_BYTES + S::B_BYTES, &map_dx, tok0, 4 * st, full_b(s));
-                if (KIND == FK_Q4_K) tma_load_2d(sa + S::A_BYTES + S::B_BYTES + S::DX_BYTES, &map_sx, tok0, 4 * st, full_b(s));
-                if (KIND == FK_Q8_0) tma_load_3d(sa, &map_w, st * KSTAGE, wrow0, mat, full_b(s));   // [matrix][row][k]: rows past a matrix's end read as zeros
+                tma_load_2d(sa + S::A_BYTES, &map_q, (st0 + st) * KSTAGE, tok0, full_b(s));
+                tma_load_2d(sa + S::A_BYTES + S::B_BYTES, &map_dx, tok0, 4 * (st0 + st), full_b(s));
+                if (KIND == FK_Q4_K) tma_load_2d(sa + S::A_BYTES + S::B_BYTES + S::DX_BYTES, &map_sx, tok0, 4 * (st0 + st), full_b(s));
+                if (KIND == FK_Q8_0) tma_load_3d(sa, &map_w, (st0 + st) * KSTAGE, wrow0, mat, full_b(s));   // [matrix][row][k]: rows past a matrix's end read as zeros
             }
         }
     } else {
@@ -461,14 +473,15 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap map_q, const _
                 const uint64_t da = umma_desc(sa), db = umma_desc(sa + S::A_BYTES);
                 for (int j = 0; j < 4; j++) {
                     const int kb = 4 * st + j;
-                    if (kb >= nkb) break;
-                    const int buf = kb % S::NACC;
-                    if (kb >= S::NACC) mbar_wait(acc_empty(buf), ((kb / S::NACC) - 1) & 1, a.err, 42);
-                    tc_fence_after();
+                    if (kb >= nkl) break;
+                    if (kb % G == 0) {
+                        if (kb >= NACC) mbar_wait(acc_empty((kb / G) & 1), ((kb / NACC) - 1) & 1, a.err, 42);
+                        tc_fence_after();
+                    }
                     // K advances 32 bytes inside the 128-byte swizzle atom: +2 in the 16-byte address field
                     GTR(0, kb, true);
-                    tc_mma_i8(tmem_base + buf * BN, da + 2 * j, db + 2 * j, IDESC);
-                    tc_commit(acc_full(buf));
+                    tc_mma_i8(tmem_base + (kb % NACC) * BN, da + 2 * j, db + 2 * j, IDESC);
+                    if (kb % G == G - 1 || kb == nkl - 1) tc_commit(acc_full((kb / G) & 1));
                 }
                 tc_commit(empty(s));   // arrives once the MMAs that read this stage are done
             }
@@ -476,40 +489,43 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap map_q, const _
     }
     tc_fence_before();
     __syncthreads();
+    if (split > 1) {
+        // the parts of the tile meet through distributed shared memory: CTA `rank` adds up its share of the token columns,
+        // in rank order (the same order whatever the timing), and writes it out
+        cluster_sync_all();
+        if (warp < EPI_WARPS) {
+            const int cols_mine = BN / split;
+            for (int i = threadIdx.x; i < cols_mine * BM; i += EPI_WARPS * 32) {
+                const int r = i & (BM - 1), c = rank * cols_mine + i / BM;
+                float pz[MAX_SPLIT];
+#pragma unroll
+                for (int z = 0; z < MAX_SPLIT; z++) pz[z] = z < split ? ld_cluster_f32(sbase + (uint32_t)(c * BM + r) * 4u, z) : 0.0f;
+                float v0 = pz[0];
+#pragma unroll
+                for (int z = 1; z < MAX_SPLIT; z++) v0 += pz[z];
+                if (KIND == FK_Q6_K) v0 += __shfl_xor_sync(0xffffffffu, v0, 1);
+                const int orow = KIND == FK_Q6_K ? wrow0 + (r >> 1) : wrow0 + r;
+                const int dst = out_row_of(tok0 + c);
+                if (orow < a.rows && (KIND != FK_Q6_K || !(r & 1)) && dst >= 0) a.out[(size_t)dst * a.rows + orow] = v0;
+            }
+        }
+        cluster_sync_all();     // no CTA leaves while another may still read its part
+    }
     if (warp == EPI_WARPS + UNPACK_WARPS + 1) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(NACC * BN) : "memory");
     }
 }
 
 // ---------------------------------------------------------------------------
-// Activation plan: q8_1 of every (padded) token row into an int8 plane
-// [n_pad][kpad] (row-major, K inner; MXFP4 keeps each run as (j, j+16) pairs)
-// plus run-major scale planes dx[nkb][n_pad] and, for Q4_K, sx = dx * run sum.
-__global__ void quantize_acts_kernel(const float* __restrict__ x, const int* __restrict__ src_row, int n_pad, int cols, int kind,
-                                     int8_t* __restrict__ q, float* __restrict__ dx, float* __restrict__ sx) {
-    const int nkb = cols >> 5;
-    const long long run = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (run >= (long long)n_pad * nkb) return;
-    const int t = (int)(run / nkb), kb = (int)(run - (long long)t * nkb);
-    const int src = src_row[t];
-    const float v = src >= 0 ? x[(size_t)src * cols + kb * 32 + lane] : 0.0f;
-    float d;
-    int qsum;
-    const int qv = fk_q8_1_lane(v, &d, &qsum);
-    const int pos = kind == FK_MXFP4 ? (((lane & 15) << 1) | (lane >> 4)) : lane;
-    q[(size_t)t * cols + kb * 32 + pos] = (int8_t)qv;
-    if (lane == 0) {
-        dx[(size_t)kb * n_pad + t] = d;
-        if (sx) sx[(size_t)kb * n_pad + t] = d * (float)qsum;
-    }
-}
-
-// The same for the kinds whose int8 plane keeps the elements in order (all but MXFP4): a thread takes four values, eight
-// lanes make a run, rows past the live tiles (`*n_tiles_dev * bn`, grouped form) are left alone -- no tile reads them.
-__global__ void quantize_acts4_kernel(const float* __restrict__ x, const int* __restrict__ src_row, int n_pad, int cols, int8_t* __restrict__ q,
+// Activation plan: q8_1 of every (padded) token row into an int8 plane [n_pad][cols] (row-major, K inner; MXFP4 keeps
+// each run as (j, j+16) pairs) plus run-major scale planes dx[nkb][n_pad] and, for Q4_K, sx = dx * run sum.  A thread
+// takes four values, eight lanes make a run.  Rows past the live tiles (`*n_tiles_dev * bn`, grouped form) are left
+// alone: no tile reads them.  src_row == nullptr (dense): row t reads token t, rows from m on are padding.
+template <bool PAIRS>
+__global__ void quantize_acts4_kernel(const float* __restrict__ x, const int* __restrict__ src_row, int m, int n_pad, int cols, int8_t* __restrict__ q,
                                       float* __restrict__ dx, float* __restrict__ sx, const int* __restrict__ n_tiles_dev, int bn) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the GEMM may set itself up and fetch weights meanwhile
     const int nkb = cols >> 5;
     const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long run = gid >> 3;
@@ -517,7 +533,7 @@ __global__ void quantize_acts4_kernel(const float* __restrict__ x, const int* __
     const int n_live = n_tiles_dev ? min(n_pad, *n_tiles_dev * bn) : n_pad;
     const bool ok = run < (long long)n_live * nkb;          // whole groups of eight lanes are in or out
     const int t = ok ? (int)(run / nkb) : 0, kb = ok ? (int)(run - (long long)t * nkb) : 0;
-    const int src = ok ? src_row[t] : -1;
+    const int src = !ok ? -1 : src_row ? src_row[t] : (t < m ? t : -1);
     float4 f = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (src >= 0) f = __ldg((const float4*)(x + (size_t)src * cols + kb * 32) + part);
     unsigned mb = __float_as_uint(fmaxf(fmaxf(fabsf(f.x), fabsf(f.y)), fmaxf(fabsf(f.z), fabsf(f.w))));
@@ -534,22 +550,17 @@ __global__ void quantize_acts4_kernel(const float* __restrict__ x, const int* __
     qsum += __shfl_xor_sync(0xffffffffu, qsum, 1);
     qsum += __shfl_xor_sync(0xffffffffu, qsum, 2);
     qsum += __shfl_xor_sync(0xffffffffu, qsum, 4);
+    const uint32_t mine = (uint32_t)(q0 & 0xFF) | ((uint32_t)(q1 & 0xFF) << 8) | ((uint32_t)(q2 & 0xFF) << 16) | ((uint32_t)(q3 & 0xFF) << 24);
+    const uint32_t other = PAIRS ? __shfl_xor_sync(0xffffffffu, mine, 4) : 0u;      // elements 16 further on (lanes 0..3 of the run)
     if (!ok) return;
-    *(uint32_t*)(q + (size_t)t * cols + kb * 32 + part * 4) =
-        (uint32_t)(q0 & 0xFF) | ((uint32_t)(q1 & 0xFF) << 8) | ((uint32_t)(q2 & 0xFF) << 16) | ((uint32_t)(q3 & 0xFF) << 24);
+    if (!PAIRS)
+        *(uint32_t*)(q + (size_t)t * cols + kb * 32 + part * 4) = mine;
+    else if (part < 4)
+        *(uint2*)(q + (size_t)t * cols + kb * 32 + part * 8) = make_uint2(__byte_perm(mine, other, 0x5140), __byte_perm(mine, other, 0x7362));
     if (part == 0) {
         const float dq = fk_h2f(fk_f2h(d));
         dx[(size_t)kb * n_pad + t] = dq;
         if (sx) sx[(size_t)kb * n_pad + t] = dq * (float)qsum;
-    }
-}
-
-// Dense plan: padded row t reads token t (t < m) and writes output row t.
-__global__ void dense_plan_kernel(int m, int n_pad, int* src_row, int* out_row) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < n_pad) {
-        src_row[t] = t < m ? t : -1;
-        out_row[t] = t < m ? t : -1;
     }
 }
 
@@ -649,76 +660,111 @@ int launch_gemm(fk_ctx* ctx, cudaStream_t st, const GemmArgs& a, const CUtensorM
     constexpr int SMEM = Smem<BN>::TOTAL;
     FK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM), FK_KERNEL);
     constexpr int WROWS = KIND == FK_Q6_K ? BM / 2 : BM;
-    dim3 grid((a.rows + WROWS - 1) / WROWS, n_token_tiles);
-    kern<<<grid, gemm_threads(BN), SMEM, st>>>(a, mq, mdx, msx, mw);
-    FK_CUDA(cudaGetLastError(), FK_LAUNCH);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((a.rows + WROWS - 1) / WROWS, n_token_tiles, a.split);
+    cfg.blockDim = dim3(Tile<BN>::THREADS);
+    cfg.dynamicSmemBytes = SMEM;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;    // set up and fetch weights while the quantizer runs
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 1;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = a.split;
+    cfg.attrs = attr;
+    cfg.numAttrs = a.split > 1 ? 2 : 1;
+    FK_CUDA(cudaLaunchKernelEx(&cfg, kern, a, mq, mdx, msx, mw), FK_LAUNCH);
     ctx->launches++;
     return FK_OK;
 }
 
 template <int BN>
-int launch_by_kind(fk_ctx* ctx, cudaStream_t st, const GemmArgs& a, const CUtensorMap& mq, const CUtensorMap& mdx, const CUtensorMap& msx,
+int launch_by_kind(fk_ctx* ctx, cudaStream_t st, const GemmArgs& a, int kind, const CUtensorMap& mq, const CUtensorMap& mdx, const CUtensorMap& msx,
                    const CUtensorMap& mw, int n_token_tiles) {
-    if (a.isums && BN == 128) {
-        switch (a.kind) {
-            case FK_Q4_K: return launch_gemm<FK_Q4_K, 128, true>(ctx, st, a, mq, mdx, msx, mw, n_token_tiles);
-            case FK_Q6_K: return launch_gemm<FK_Q6_K, 128, true>(ctx, st, a, mq, mdx, msx, mw, n_token_tiles);
-            case FK_Q8_0: return launch_gemm<FK_Q8_0, 128, true>(ctx, st, a, mq, mdx, msx, mw, n_token_tiles);
-            case FK_MXFP4: return launch_gemm<FK_MXFP4, 128, true>(ctx, st, a, mq, mdx, msx, mw, n_token_tiles);
+    if (a.isums) {
+        switch (kind) {
+            case FK_Q4_K: return launch_gemm<FK_Q4_K, BN, true>(ctx, st, a, mq, mdx, msx, mw, n_token_tiles);
+            case FK_Q6_K: return launch_gemm<FK_Q6_K, BN, true>(ctx, st, a, mq, mdx, msx, mw, n_token_tiles);
+            case FK_Q8_0: return launch_gemm<FK_Q8_0, BN, true>(ctx, st, a, mq, mdx, msx, mw, n_token_tiles);
+            case FK_MXFP4: return launch_gemm<FK_MXFP4, BN, true>(ctx, st, a, mq, mdx, msx, mw, n_token_tiles);
         }
     }
-    switch (a.kind) {
+    switch (kind) {
         case FK_Q4_K: return launch_gemm<FK_Q4_K, BN>(ctx, st, a, mq, mdx, msx, mw, n_token_tiles);
         case FK_Q6_K: return launch_gemm<FK_Q6_K, BN>(ctx, st, a, mq, mdx, msx, mw, n_token_tiles);
         case FK_Q8_0: return launch_gemm<FK_Q8_0, BN>(ctx, st, a, mq, mdx, msx, mw, n_token_tiles);
         case FK_MXFP4: return launch_gemm<FK_MXFP4, BN>(ctx, st, a, mq, mdx, msx, mw, n_token_tiles);
     }
-    return fk_fail(FK_UNSUPPORTED, "gemm: kind %d has no kernel", a.kind);
+    return fk_fail(FK_UNSUPPORTED, "gemm: kind %d has no kernel", kind);
 }
 
-// Shared body of fk_gemm (group_off == nullptr) and fk_gemm_grouped.
-int gemm_common(fk_ctx* ctx, cudaStream_t st, fk_weight w, int mat, const int* group_off, const int* gather, const float* x,
-                int n_tokens, float* out, int32_t* isums = nullptr) {
-    const bool grouped = group_off != nullptr;
-    if (w->kind == FK_Q5_K || w->kind == FK_BF16)   // before anything is enqueued: the caller takes batches of 8 through the matvec
-        return fk_fail(FK_UNSUPPORTED, "gemm: kind %d has the plain matvec only", w->kind);
-    const int bn = grouped ? 64 : 128;
-    const int n_tiles_max = grouped ? (n_tokens + bn - 1) / bn + w->n_mats : (n_tokens + bn - 1) / bn;
-    const int n_pad = n_tiles_max * bn;
-    const int nkb = w->cols / 32;
-    // scratch: q plane | dx | sx | src_row | out_row | tile_expert | n_tiles
-    size_t off_q = 0, off_dx = align_up(off_q + (size_t)n_pad * w->cols, 1024);
-    size_t off_sx = align_up(off_dx + (size_t)nkb * n_pad * 4, 1024);
-    size_t off_src = align_up(off_sx + (size_t)nkb * n_pad * 4, 1024);
-    size_t off_out = off_src + (size_t)n_pad * 4, off_te = off_out + (size_t)n_pad * 4;
-    size_t off_nt = off_te + (size_t)n_tiles_max * 4, total = off_nt + 16;
-    int rc = fk_ensure_scratch(ctx, st, total);
-    if (rc) return rc;
-    uint8_t* sc = ctx->scratch;
-    int8_t* q = (int8_t*)(sc + off_q);
-    float* dx = (float*)(sc + off_dx);
-    float* sx = (float*)(sc + off_sx);
-    int* src_row = (int*)(sc + off_src);
-    int* out_row = (int*)(sc + off_out);
-    int* tile_expert = (int*)(sc + off_te);
-    int* n_tiles = (int*)(sc + off_nt);
+// Which tile (token columns per CTA) and how many CTAs along K: the candidate with the smallest estimated time
+//
+//   waves * (runs / split * us_per_run(bn) + (split > 1) * exchange(bn)),   waves = CTAs / (SMs * CTAs per SM)
+//
+// The constants were measured on B200 (us; Q4_K, 3072 x 3072, cold L2; the other kinds are within 15 %): a 128-token tile
+// takes 0.82 a run of 32 K, a 64-token one 0.47, a 32-token one 0.40 alone on its SM and 0.56 beside another; the parts of
+// a split tile take 6 to 9 to meet.  A tile's own time hardly falls with its width -- its warps walk the same chain per
+// run -- so what a short prompt needs is more CTAs, not narrower ones: 3072 x 3072, M = 128 was 24 CTAs and 95 us, and is
+// 96 CTAs and 36 us; 3072 x 8192 Q6_K, M = 77 204 -> 81 us; 512 x 3072, M = 16 93 -> 17 us; 8192 x 3072, M = 512 keeps
+// whole 128-token tiles (167 us; 64-token tiles 185, 32-token ones 200).  Grouped: `tiles` expects half a tile of padding
+// per expert, which is what 32-token tiles win by (128 experts, 8 of them for each of 77 rows, 768 x 2048 Q4_K: the routed
+// layer takes 486 us against 763 with 64-token tiles and 1226 with 128).
+struct GemmPlan { int bn, split; };
 
-    if (grouped) {
-        grouped_plan_kernel<<<1, 1024, 2 * (w->n_mats + 1) * sizeof(int), st>>>(group_off, gather, w->n_mats, bn, n_pad, src_row, out_row,
-                                                                             tile_expert, n_tiles);
-    } else {
-        dense_plan_kernel<<<(n_pad + 255) / 256, 256, 0, st>>>(n_tokens, n_pad, src_row, out_row);
+GemmPlan gemm_plan(const fk_ctx* ctx, const fk_weight_s* w, int m, bool grouped) {
+    const int wrows = w->kind == FK_Q6_K ? BM / 2 : BM, row_tiles = (w->rows + wrows - 1) / wrows;
+    const int runs = w->cols / 32, stages = (runs + 3) / 4;
+    GemmPlan best{128, 1};
+    double best_us = 1e30;
+    for (int bn : {128, 64, 32}) {
+        const double tiles = grouped ? (double)m / bn + 0.5 * (m < w->n_mats ? m : w->n_mats) : (double)((m + bn - 1) / bn);
+        for (int split = 1; split <= MAX_SPLIT && split <= stages; split *= 2) {
+            const double ctas = tiles * row_tiles * split;
+            const double sms = split == 8 ? 0.9 * ctx->sm_count : ctx->sm_count;       // clusters of eight do not tile every GPC
+            const bool two = bn == 32 && ctas > sms;
+            double us = bn == 128 ? (w->kind == FK_MXFP4 ? 1.03 : 0.82) : bn == 64 ? 0.47 : two ? 0.56 : 0.40;
+            us = us * (4 * ((stages + split - 1) / split)) + (split > 1 ? (bn == 128 ? 9.0 : bn == 64 ? 7.0 : 6.0) : 0.0);
+            const double waves = ctas / (two ? 2.0 * sms : sms);
+            us *= waves > 4.0 ? waves + 0.25 : ceil(waves);
+            if (us < best_us) { best_us = us; best = {bn, split}; }
+        }
     }
-    FK_CUDA(cudaGetLastError(), FK_LAUNCH);
-    const long long runs = (long long)n_pad * nkb;
-    if (w->kind == FK_MXFP4)
-        quantize_acts_kernel<<<(unsigned)((runs + 7) / 8), 256, 0, st>>>(x, src_row, n_pad, w->cols, w->kind, q, dx, nullptr);
-    else
-        quantize_acts4_kernel<<<(unsigned)((runs + 31) / 32), 256, 0, st>>>(x, src_row, n_pad, w->cols, q, dx, w->kind == FK_Q4_K ? sx : nullptr,
-                                                                            grouped ? n_tiles : nullptr, bn);
-    FK_CUDA(cudaGetLastError(), FK_LAUNCH);
-    ctx->launches += 2;
+    return best;
+}
 
+// The scratch of one call: q plane | dx | sx | row tables of the grouped form.
+struct GemmScratch {
+    size_t dx, sx, src, out, te, nt, total;
+    GemmScratch(int n_pad, int cols, int n_tiles, bool grouped) {
+        const int nkb = cols / 32;
+        dx = align_up((size_t)n_pad * cols, 1024);
+        sx = align_up(dx + (size_t)nkb * n_pad * 4, 1024);
+        src = align_up(sx + (size_t)nkb * n_pad * 4, 1024);
+        out = src + (grouped ? (size_t)n_pad * 4 : 0);
+        te = out + (grouped ? (size_t)n_pad * 4 : 0);
+        nt = te + (grouped ? (size_t)n_tiles * 4 : 0);
+        total = nt + 16;
+    }
+};
+
+// Quantizer and GEMM of one call on a prepared scratch block (fk_gemm, fk_gemm_grouped after its plan, fk_gemm_static).
+int gemm_run(fk_ctx* ctx, cudaStream_t st, fk_weight w, int mat, const float* x, int m, float* out, int32_t* isums, const GemmPlan& plan,
+             uint8_t* sc, const GemmScratch& L, int n_pad, bool grouped) {
+    const int bn = plan.bn, nkb = w->cols / 32;
+    int8_t* q = (int8_t*)sc;
+    float *dx = (float*)(sc + L.dx), *sx = (float*)(sc + L.sx);
+    const int* src_row = grouped ? (const int*)(sc + L.src) : nullptr;
+    const int* n_tiles = grouped ? (const int*)(sc + L.nt) : nullptr;
+    const unsigned qgrid = (unsigned)(((long long)n_pad * nkb + 31) / 32);
+    float* sxq = w->kind == FK_Q4_K ? sx : nullptr;
+    if (w->kind == FK_MXFP4) quantize_acts4_kernel<true><<<qgrid, 256, 0, st>>>(x, src_row, m, n_pad, w->cols, q, dx, sxq, n_tiles, bn);
+    else quantize_acts4_kernel<false><<<qgrid, 256, 0, st>>>(x, src_row, m, n_pad, w->cols, q, dx, sxq, n_tiles, bn);
+    FK_CUDA(cudaGetLastError(), FK_LAUNCH);
+    ctx->launches++;
+
+    int rc;
     CUtensorMap mq, mdx, msx, mw;
     if ((rc = make_map(&mq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, q, w->cols, n_pad, KSTAGE, bn, CU_TENSOR_MAP_SWIZZLE_128B))) return rc;
     if ((rc = make_map(&mdx, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, dx, n_pad, nkb, bn, 4, CU_TENSOR_MAP_SWIZZLE_NONE))) return rc;
@@ -729,17 +775,42 @@ int gemm_common(fk_ctx* ctx, cudaStream_t st, fk_weight w, int mat, const int* g
     a.w = w->dev;
     a.mat_stride = w->mat_stride;
     for (int i = 0; i < 4; i++) { a.plane_off[i] = w->plane_off[i]; a.plane_stride[i] = w->plane_stride[i]; }
-    a.kind = w->kind;
     a.rows = w->rows;
     a.cols = w->cols;
     a.mat = mat;
-    a.tile_expert = grouped ? tile_expert : nullptr;
-    a.n_tiles_dev = grouped ? n_tiles : nullptr;
-    a.out_row = out_row;
+    a.tile_expert = grouped ? (const int*)(sc + L.te) : nullptr;
+    a.n_tiles_dev = n_tiles;
+    a.out_row = grouped ? (const int*)(sc + L.out) : nullptr;
+    a.m = m;
+    a.split = plan.split;
     a.out = out;
     a.isums = isums;
     a.err = ctx->err_flag;
-    return grouped ? launch_by_kind<64>(ctx, st, a, mq, mdx, msx, mw, n_tiles_max) : launch_by_kind<128>(ctx, st, a, mq, mdx, msx, mw, n_tiles_max);
+    const int tiles = n_pad / bn;
+    return bn == 128  ? launch_by_kind<128>(ctx, st, a, w->kind, mq, mdx, msx, mw, tiles)
+           : bn == 64 ? launch_by_kind<64>(ctx, st, a, w->kind, mq, mdx, msx, mw, tiles)
+                      : launch_by_kind<32>(ctx, st, a, w->kind, mq, mdx, msx, mw, tiles);
+}
+
+// Shared body of fk_gemm (group_off == nullptr) and fk_gemm_grouped.
+int gemm_common(fk_ctx* ctx, cudaStream_t st, fk_weight w, int mat, const int* group_off, const int* gather, const float* x,
+                int n_tokens, float* out, int32_t* isums = nullptr) {
+    const bool grouped = group_off != nullptr;
+    if (w->kind == FK_Q5_K || w->kind == FK_BF16)   // before anything is enqueued: the caller takes batches of 8 through the matvec
+        return fk_fail(FK_UNSUPPORTED, "gemm: kind %d has the plain matvec only", w->kind);
+    const GemmPlan plan = gemm_plan(ctx, w, n_tokens, grouped);
+    const int n_tiles_max = (n_tokens + plan.bn - 1) / plan.bn + (grouped ? w->n_mats : 0), n_pad = n_tiles_max * plan.bn;
+    const GemmScratch L(n_pad, w->cols, n_tiles_max, grouped);
+    int rc = fk_ensure_scratch(ctx, st, L.total);
+    if (rc) return rc;
+    uint8_t* sc = ctx->scratch;
+    if (grouped) {
+        grouped_plan_kernel<<<1, 1024, 2 * (w->n_mats + 1) * sizeof(int), st>>>(group_off, gather, w->n_mats, plan.bn, n_pad, (int*)(sc + L.src),
+                                                                             (int*)(sc + L.out), (int*)(sc + L.te), (int*)(sc + L.nt));
+        FK_CUDA(cudaGetLastError(), FK_LAUNCH);
+        ctx->launches++;
+    }
+    return gemm_run(ctx, st, w, mat, x, n_tokens, out, isums, plan, sc, L, n_pad, grouped);
 }
 
 }  // namespace
@@ -828,53 +899,20 @@ FK_EXPORT int fk_gemm_static(fk_ctx* ctx, void* stream, fk_weight w, int mat, co
     if (mat < 0 || mat >= w->n_mats) return fk_fail(FK_INVALID, "gemm_static: matrix %d of %d", mat, w->n_mats);
     FkDeviceGuard g(ctx->device);
     cudaStream_t st = (cudaStream_t)stream;
-    const int bn = 128;
-    const int n_tiles = (m + bn - 1) / bn, n_pad = n_tiles * bn, nkb = w->cols / 32;
-    // the same carve-up as fk_gemm's: q plane | dx | sx | src_row | out_row
-    const size_t off_dx = align_up((size_t)n_pad * w->cols, 1024);
-    const size_t off_sx = align_up(off_dx + (size_t)nkb * n_pad * 4, 1024);
-    const size_t off_src = align_up(off_sx + (size_t)nkb * n_pad * 4, 1024);
-    const size_t off_out = off_src + (size_t)n_pad * 4, total = off_out + (size_t)n_pad * 4;
-    if (total > FK_GEMM_STATIC_BYTES)
+    if (w->kind == FK_Q5_K || w->kind == FK_BF16) return fk_fail(FK_UNSUPPORTED, "gemm: kind %d has no kernel", w->kind);
+    // Sized for tiles of 128 tokens whatever tile the plan picks (narrower ones pad less): what fits does not depend on it.
+    const GemmScratch most((m + 127) / 128 * 128, w->cols, 0, false);
+    if (most.total > FK_GEMM_STATIC_BYTES)
         return fk_fail(FK_INVALID, "gemm_static: %d tokens x %d columns needs %zu bytes of scratch, the fixed block holds %zu (use fk_gemm)",
-                       m, w->cols, total, (size_t)FK_GEMM_STATIC_BYTES);
+                       m, w->cols, most.total, (size_t)FK_GEMM_STATIC_BYTES);
     uint8_t* sc = nullptr;
     int rc = static_scratch(ctx, &sc);
     if (rc) return rc;
-    int8_t* q = (int8_t*)sc;
-    float* dx = (float*)(sc + off_dx);
-    float* sx = (float*)(sc + off_sx);
-    int* src_row = (int*)(sc + off_src);
-    int* out_row = (int*)(sc + off_out);
-    // Nothing in the block has to start at zero: the two kernels below write every
-    // word the GEMM reads (padding rows included) before it reads them.
-    dense_plan_kernel<<<(n_pad + 255) / 256, 256, 0, st>>>(m, n_pad, src_row, out_row);
-    FK_CUDA(cudaGetLastError(), FK_LAUNCH);
-    const long long runs = (long long)n_pad * nkb;
-    quantize_acts_kernel<<<(unsigned)((runs + 7) / 8), 256, 0, st>>>(x_dev, src_row, n_pad, w->cols, w->kind, q, dx, w->kind == FK_Q4_K ? sx : nullptr);
-    FK_CUDA(cudaGetLastError(), FK_LAUNCH);
-    ctx->launches += 2;
-    CUtensorMap mq, mdx, msx, mw;
-    if ((rc = make_map(&mq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, q, w->cols, n_pad, KSTAGE, bn, CU_TENSOR_MAP_SWIZZLE_128B))) return rc;
-    if ((rc = make_map(&mdx, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, dx, n_pad, nkb, bn, 4, CU_TENSOR_MAP_SWIZZLE_NONE))) return rc;
-    if ((rc = make_map(&msx, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, sx, n_pad, nkb, bn, 4, CU_TENSOR_MAP_SWIZZLE_NONE))) return rc;
-    mw = mq;
-    if (w->kind == FK_Q8_0 && (rc = make_map_q8_0(&mw, w))) return rc;
-    GemmArgs a;
-    a.w = w->dev;
-    a.mat_stride = w->mat_stride;
-    for (int i = 0; i < 4; i++) { a.plane_off[i] = w->plane_off[i]; a.plane_stride[i] = w->plane_stride[i]; }
-    a.kind = w->kind;
-    a.rows = w->rows;
-    a.cols = w->cols;
-    a.mat = mat;
-    a.tile_expert = nullptr;
-    a.n_tiles_dev = nullptr;
-    a.out_row = out_row;
-    a.out = out_dev;
-    a.isums = nullptr;
-    a.err = ctx->err_flag;
-    return launch_by_kind<128>(ctx, st, a, mq, mdx, msx, mw, n_tiles);
+    // Nothing in the block has to start at zero: the quantizer writes every word the GEMM reads (padding rows included)
+    // before it reads them.
+    const GemmPlan plan = gemm_plan(ctx, w, m, false);
+    const int n_pad = (m + plan.bn - 1) / plan.bn * plan.bn;
+    return gemm_run(ctx, st, w, mat, x_dev, m, out_dev, nullptr, plan, sc, GemmScratch(n_pad, w->cols, 0, false), n_pad, false);
 }
 
 // The error word kernels raise when a bounded wait gives up: 0 = none.
