@@ -10,7 +10,7 @@
 // is drained from tensor memory after every K = 32 step and scaled on the CUDA
 // cores; that rescale, not the tensor pipe, bounds this kernel.  Accumulators change hands in groups (half of tensor
 // memory at a time), not run by run, and the launch overlaps the quantizer in front of it (programmatic serialization):
-// with the decode of the weight scales moved off their load, 8192 x 3072, M = 512 went from 185 to 167 us.
+// with the weight scales decoded by the unpack warps, 8192 x 3072, M = 512 went from 185 to 142 us.
 //
 // One CTA = 128 weight rows x BN tokens (128, 64 or 32; gemm_plan), warps with fixed roles (Tile<BN>):
 //   epilogue    TMEM -> registers (tcgen05.ld), f32 rescale, store
@@ -81,15 +81,18 @@ template <int BN> struct Smem {
     static constexpr int A_BYTES = BM * KSTAGE;          // 16 KB
     static constexpr int B_BYTES = BN * KSTAGE;
     static constexpr int DX_BYTES = 4 * BN * 4;          // [4 runs][BN] f32
-    static constexpr int STAGE = A_BYTES + B_BYTES + 2 * DX_BYTES;
+    static constexpr int DW_BYTES = 4 * BM * 4;          // [4 runs][BM] f32: weight scales, then (Q4_K) min scales
+    static constexpr int DX = A_BYTES + B_BYTES, DW = DX + 2 * DX_BYTES;
+    static constexpr int STAGE = DW + 2 * DW_BYTES;
     static constexpr int BARS = NSTAGE * STAGE;          // barrier block
     static constexpr int TOTAL = BARS + 256 + 1024;      // + alignment slack
     static_assert(BM * BN * 4 <= BARS, "the partial sums of a split tile reuse the stages");
 };
 
-// The weight scales of one tile row for one stage (runs kb0 .. kb0 + 3): as loaded, and decoded.  The load is issued a
-// stage ahead and nothing touches its registers until that stage begins -- decoding at the load, as this once did, made
-// every warp wait out a global-memory latency per stage (2000 of 7600 cycles of a 128-token tile).
+// The weight scales of one tile row for one stage (runs kb0 .. kb0 + 3): as loaded, and decoded.  The unpack warps load
+// them beside the row they belong to and leave them decoded in the stage, so the epilogue -- the kernel's critical path --
+// reads one or two words a run.  (Loaded by every epilogue warp for itself they cost each stage a global-memory latency:
+// 340 to 1800 cycles out of 2400 to 7000.)
 template <int KIND> struct RawScale {
     uint4 hd;        // Q4_K: d, dmin and the packed scales
     uint2 sc;        // Q8_0: four f16; Q6_K: eight int8 (two per run); MXFP4: four exponents in x
@@ -98,24 +101,22 @@ template <int KIND> struct RawScale {
 struct StageScale { uint32_t sc, mn; float d, dmin; uint2 raw; };
 
 template <int KIND>
-__device__ __forceinline__ RawScale<KIND> load_wscales(const GemmArgs& a, const uint8_t* wb, int row, bool row_ok, int kb0) {
-    RawScale<KIND> v;
+__device__ __forceinline__ void load_wscales(const GemmArgs& a, const uint8_t* wb, int wrow0, int r, int st, bool live, RawScale<KIND>& v) {
     v.hd = make_uint4(0, 0, 0, 0);
     v.sc = make_uint2(0, 0);
     v.d = 0;
-    if (!row_ok) return v;
+    const int kb0 = 4 * st, wrow = wrow0 + (KIND == FK_Q6_K ? r >> 1 : r);
+    if (!live || wrow >= a.rows) return;
     if (KIND == FK_Q4_K) {
-        v.hd = ldg16(wb + ((size_t)row * (a.cols >> 8) + (kb0 >> 3)) * 144);
+        v.hd = ldg16(wb + ((size_t)wrow * (a.cols >> 8) + (kb0 >> 3)) * 144);
     } else if (KIND == FK_Q8_0) {
-        v.sc = __ldg((const uint2*)(wb + a.plane_off[1] + (size_t)row * a.plane_stride[1] + 2 * kb0));   // rows are padded to 16 bytes
+        v.sc = __ldg((const uint2*)(wb + a.plane_off[1] + (size_t)wrow * a.plane_stride[1] + 2 * kb0));   // rows are padded to 16 bytes
     } else if (KIND == FK_MXFP4) {
-        v.sc.x = __ldg((const uint32_t*)(wb + a.plane_off[1] + (size_t)row * a.plane_stride[1] + kb0));
-    } else {  // FK_Q6_K: `row` = 2 * weight row + half
-        const int wrow = row >> 1;
+        v.sc.x = __ldg((const uint32_t*)(wb + a.plane_off[1] + (size_t)wrow * a.plane_stride[1] + kb0));
+    } else {
         v.d = __ldg((const uint16_t*)(wb + a.plane_off[3] + (size_t)wrow * a.plane_stride[3]) + (kb0 >> 3));
         v.sc = __ldg((const uint2*)(wb + a.plane_off[2] + (size_t)wrow * a.plane_stride[2] + 2 * kb0));
     }
-    return v;
 }
 template <int KIND>
 __device__ __forceinline__ StageScale stage_scales(const RawScale<KIND>& v, int kb0) {
@@ -230,6 +231,11 @@ __device__ __forceinline__ void store_raw(const RawRow<KIND>& raw, int r, uint8_
     for (int c = 0; c < 8; c++) *(uint4*)(dst + ((c ^ (r & 7)) << 4)) = o[c];
 }
 
+__device__ __forceinline__ float lds32f(uint32_t addr) {
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+    return v;
+}
 __device__ __forceinline__ float ld_cluster_f32(uint32_t addr, int rank) {
     uint32_t remote;
     float v;
@@ -247,7 +253,7 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap map_q, const _
             const __grid_constant__ CUtensorMap map_sx, const __grid_constant__ CUtensorMap map_w) {
     using S = Smem<BN>;
     using T = Tile<BN>;
-    constexpr int EPI_WARPS = T::EPI_WARPS, UNPACK_WARPS = T::UNPACK_WARPS, NACC = T::NACC, G = T::GROUP, CW = T::CW, HC = CW / 2;
+    constexpr int EPI_WARPS = T::EPI_WARPS, UNPACK_WARPS = T::UNPACK_WARPS, NACC = T::NACC, G = T::GROUP, CW = T::CW, NCH = CW / 16;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const uint32_t sbase = smem_u32(smem);
@@ -308,7 +314,6 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap map_q, const _
         // ------------------------------------------------------------ epilogue
         const int quad = warp & 3, chalf = warp >> 2;
         const int r = quad * 32 + lane;                // tile row = TMEM lane
-        const int row = KIND == FK_Q6_K ? 2 * wrow0 + r : wrow0 + r;   // scale row id (pair id for Q6_K)
         const bool row_ok = (KIND == FK_Q6_K ? (wrow0 + (r >> 1)) : (wrow0 + r)) < a.rows;
         const int orow = KIND == FK_Q6_K ? wrow0 + (r >> 1) : wrow0 + r;
         const bool writer = row_ok && (KIND != FK_Q6_K || !(r & 1));
@@ -316,84 +321,83 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap map_q, const _
 #pragma unroll
         for (int i = 0; i < CW; i++) acc[i] = 0.0f;
         const uint32_t taddr0 = tmem_base + ((uint32_t)(quad * 32) << 16) + chalf * CW;
-        RawScale<KIND> ws_next = load_wscales<KIND>(a, wb, row, row_ok, kb_lo);
         if (!a.n_tiles_dev) asm volatile("griddepcontrol.wait;" ::: "memory");
-        // TMEM reads are double-buffered in halves of HC columns: while one half is
-        // scaled the next one (or the next run's first) is already in flight, so a warp's
-        // chain per run is its arithmetic, not the accumulator hand-off latency.
-        uint32_t v[2][HC];
+        // TMEM reads are double-buffered in chunks of 16 columns (two a run, or one): while one chunk is scaled the next is
+        // already in flight, so a warp's chain per run is its arithmetic, not the accumulator hand-off latency.
+        uint32_t va[16], vb[16];
         auto issue = [&](int kb, int c, uint32_t* dst) {   // kb counts from this CTA's first run
             if (c == 0 && kb % G == 0) {
                 mbar_wait(acc_full((kb / G) & 1), (kb / NACC) & 1, a.err, 11);
                 tc_fence_after();
                 GTR(1, kb, warp == 0 && lane == 0);
             }
-            if (HC == 16) tc_ld16(taddr0 + (kb % NACC) * BN + c * HC, dst);
-            else tc_ld8(taddr0 + (kb % NACC) * BN + c * HC, dst);
+            tc_ld16(taddr0 + (kb % NACC) * BN + c * 16, dst);
         };
-        issue(0, 0, v[0]);
+        issue(0, 0, va);
         tc_wait_ld();
-        tc_ld_fence<HC>(v[0]);
+        tc_ld_fence<16>(va);
+        float dw = 0.0f, mw = 0.0f;
+        // chunk c of run kb (= run j of the stage at sdx_s) out of cur, the chunk after it on its way into nxt
+        auto step = [&](int kb, int j, int c, uint32_t sdx_s, uint32_t* cur, uint32_t* nxt) {
+            const int kb_n = c == NCH - 1 ? kb + 1 : kb, c_n = c == NCH - 1 ? 0 : c + 1;
+            if (c == 0) {
+                const uint32_t sw = sdx_s + (uint32_t)(S::DW - S::DX) + (uint32_t)(j * BM + r) * 4u;
+                dw = lds32f(sw);
+                if (KIND == FK_Q4_K) mw = lds32f(sw + S::DW_BYTES);
+            }
+            if (kb_n < nkl) issue(kb_n, c_n, nxt);
+            const uint32_t dxs = sdx_s + (uint32_t)(j * BN + chalf * CW + c * 16) * 4u;
+            if (DUMP && row_ok) {
+                // the exact integers of this run, before any scale touches them
+                const int nruns = KIND == FK_Q6_K ? a.cols >> 4 : nkb, run = KIND == FK_Q6_K ? 2 * (kb_lo + kb) + (r & 1) : kb_lo + kb;
+                for (int i = 0; i < 16; i++) {
+                    const int dst = out_row_of(tok0 + chalf * CW + c * 16 + i);
+                    if (dst >= 0) a.isums[((size_t)dst * a.rows + orow) * nruns + run] = (int32_t)cur[i];
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 16; i += 4) {
+                const float4 dx = lds128(dxs + 4u * i);
+                const float dxa[4] = {dx.x, dx.y, dx.z, dx.w};
+                float sxa[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                if (KIND == FK_Q4_K) {
+                    const float4 sx = lds128(dxs + 16u * BN + 4u * i);
+                    sxa[0] = sx.x; sxa[1] = sx.y; sxa[2] = sx.z; sxa[3] = sx.w;
+                }
+                // two columns per instruction on the packed f32x2 path; int32 -> f32 (exact, |C| < 2^22) on the
+                // conversion unit: one issue slot, where the magic-number add takes two on the integer and FP32 pipes
+#pragma unroll
+                for (int e = 0; e < 4; e += 2) {
+                    const float2 f2 = make_float2((float)(int)cur[i + e], (float)(int)cur[i + e + 1]);
+                    const float2 s2 = __fmul2_rn(make_float2(dw, dw), make_float2(dxa[e], dxa[e + 1]));
+                    float2 t2 = __ffma2_rn(s2, f2, make_float2(acc[c * 16 + i + e], acc[c * 16 + i + e + 1]));
+                    if (KIND == FK_Q4_K) t2 = __ffma2_rn(make_float2(-mw, -mw), make_float2(sxa[e], sxa[e + 1]), t2);
+                    acc[c * 16 + i + e] = t2.x;
+                    acc[c * 16 + i + e + 1] = t2.y;
+                }
+            }
+            tc_wait_ld();
+            tc_ld_fence<16>(nxt);
+            if (kb_n < nkl && c_n == NCH - 1 && (kb_n % G == G - 1 || kb_n == nkl - 1)) {   // the group's last chunk is in registers: hand it back
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(acc_empty((kb_n / G) & 1));
+            }
+        };
         for (int st = 0; st < nst; st++) {
             const int s = st % NSTAGE;
-            const StageScale ws = stage_scales<KIND>(ws_next, kb_lo + 4 * st);
-            if (st + 1 < nst) ws_next = load_wscales<KIND>(a, wb, row, row_ok, kb_lo + 4 * (st + 1));
-            mbar_wait(full_b(s), (st / NSTAGE) & 1, a.err, 10);   // the scale tiles of this stage have landed
-            // the stage's scale tiles: dx [4][BN] then (Q4_K) sx [4][BN], as shared-space addresses
-            const uint32_t sdx_s = sbase + s * S::STAGE + S::A_BYTES + S::B_BYTES;
+            mbar_wait(full_a(s), (st / NSTAGE) & 1, a.err, 9);    // the scale tiles of this stage: the weights' ...
+            mbar_wait(full_b(s), (st / NSTAGE) & 1, a.err, 10);   // ... and the activations': dx [4][BN] then (Q4_K) sx [4][BN]
+            const uint32_t sdx_s = sbase + s * S::STAGE + S::DX;
             // Rolled on purpose: the unrolled body falls out of the instruction cache.
 #pragma unroll 1
-            for (int j = 0; j < 4; j++) {
-                const int kb = 4 * st + j;
+            for (int q = 0; q < 4 * NCH; q += 2) {
+                const int j = q / NCH, kb = 4 * st + j;
                 if (kb >= nkl) break;
-                float dw, mw;
-                run_scale<KIND>(ws, j, row, &dw, &mw);
-#pragma unroll
-                for (int c = 0; c < 2; c++) {
-                    uint32_t* cur = v[c];
-                    uint32_t* nxt = v[c ^ 1];
-                    const int kb_n = c == 0 ? kb : kb + 1, c_n = c ^ 1;
-                    if (kb_n < nkl) issue(kb_n, c_n, nxt);
-                    const uint32_t dxs = sdx_s + (uint32_t)(j * BN + chalf * CW + c * HC) * 4u;
-                    if (DUMP && row_ok) {
-                        // the exact integers of this run, before any scale touches them
-                        const int orow_d = KIND == FK_Q6_K ? wrow0 + (r >> 1) : wrow0 + r;
-                        const int nruns = KIND == FK_Q6_K ? a.cols >> 4 : nkb, run = KIND == FK_Q6_K ? 2 * (kb_lo + kb) + (r & 1) : kb_lo + kb;
-                        for (int i = 0; i < HC; i++) {
-                            const int dst = out_row_of(tok0 + chalf * CW + c * HC + i);
-                            if (dst >= 0) a.isums[((size_t)dst * a.rows + orow_d) * nruns + run] = (int32_t)cur[i];
-                        }
-                    }
-#pragma unroll
-                    for (int i = 0; i < HC; i += 4) {
-                        const float4 dx = lds128(dxs + 4u * i);
-                        const float dxa[4] = {dx.x, dx.y, dx.z, dx.w};
-                        float sxa[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-                        if (KIND == FK_Q4_K) {
-                            const float4 sx = lds128(dxs + 16u * BN + 4u * i);
-                            sxa[0] = sx.x; sxa[1] = sx.y; sxa[2] = sx.z; sxa[3] = sx.w;
-                        }
-                        // two columns per instruction on the packed f32x2 path; int32 -> f32 (exact, |C| < 2^22) on the
-                        // conversion unit: one issue slot, where the magic-number add takes two on the integer and FP32 pipes
-#pragma unroll
-                        for (int e = 0; e < 4; e += 2) {
-                            const float2 f2 = make_float2((float)(int)cur[i + e], (float)(int)cur[i + e + 1]);
-                            const float2 s2 = __fmul2_rn(make_float2(dw, dw), make_float2(dxa[e], dxa[e + 1]));
-                            float2 t2 = __ffma2_rn(s2, f2, make_float2(acc[c * HC + i + e], acc[c * HC + i + e + 1]));
-                            if (KIND == FK_Q4_K) t2 = __ffma2_rn(make_float2(-mw, -mw), make_float2(sxa[e], sxa[e + 1]), t2);
-                            acc[c * HC + i + e] = t2.x;
-                            acc[c * HC + i + e + 1] = t2.y;
-                        }
-                    }
-                    tc_wait_ld();
-                    tc_ld_fence<HC>(nxt);
-                    GTR(2, kb, warp == 0 && lane == 0 && c == 1);
-                    if (kb_n < nkl && c_n == 1 && (kb_n % G == G - 1 || kb_n == nkl - 1)) {   // the group's last half is in registers: hand it back
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(acc_empty((kb_n / G) & 1));
-                    }
-                }
+                step(kb, j, 0, sdx_s, va, vb);
+                if (NCH == 1 && kb + 1 >= nkl) break;
+                if (NCH == 1) step(kb + 1, j + 1, 0, sdx_s, vb, va);
+                else step(kb, j, 1, sdx_s, vb, va);
             }
             // this warp is done with the stage's scale tiles
             __syncwarp();
@@ -401,7 +405,7 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap map_q, const _
         }
         if (split == 1) {
             // ---- store: out[out_row[token]][weight row]
-#pragma unroll 4
+#pragma unroll
             for (int i = 0; i < CW; i++) {
                 float v0 = acc[i];
                 if (KIND == FK_Q6_K) v0 += __shfl_xor_sync(0xffffffffu, v0, 1);   // the two halves of a weight row sit in neighbouring lanes
@@ -418,30 +422,47 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap map_q, const _
         }
     } else if (warp < EPI_WARPS + UNPACK_WARPS) {
         // ------------------------------------------------- weight unpack warps
-        if (KIND != FK_Q8_0) {
-            // a thread owns NR tile rows; the loads of the next DEPTH stages are in flight while a stage is written
-            constexpr int NR = BM / (32 * UNPACK_WARPS), DEPTH = NR == 1 ? 2 : 1;
-            const int t = (warp - EPI_WARPS) * 32 + lane;
-            RawRow<KIND> raw[DEPTH + 1][NR];
+        // A thread owns NR tile rows (Q8_0: their scales only); the loads of the next DEPTH stages are in flight while a stage
+        // is written.  The slots are rotated by unrolling, not by copying: a register move out of a load that is still in
+        // flight waits for it, and the prefetch with it (3072 x 3072 Q4_K in 32-token tiles: 62 us with moves, 46 without).
+        constexpr int NR = BM / (32 * UNPACK_WARPS), DEPTH = BN == 64 ? 2 : 1, SLOTS = DEPTH + 1;
+        const int t = (warp - EPI_WARPS) * 32 + lane;
+        RawRow<KIND> raw[SLOTS][NR];
+        RawScale<KIND> rsc[SLOTS][NR];
+        auto load = [&](int p, int st) {
 #pragma unroll
-            for (int p = 0; p < DEPTH; p++)
+            for (int i = 0; i < NR; i++) {
+                load_raw<KIND>(a, wb, wrow0, t + 32 * UNPACK_WARPS * i, st0 + st, st < nst, raw[p][i]);
+                load_wscales<KIND>(a, wb, wrow0, t + 32 * UNPACK_WARPS * i, st0 + st, st < nst, rsc[p][i]);
+            }
+        };
 #pragma unroll
-                for (int i = 0; i < NR; i++) load_raw<KIND>(a, wb, wrow0, t + 32 * UNPACK_WARPS * i, st0 + p, p < nst, raw[p][i]);
-            for (int st = 0; st < nst; st++) {
-                const int s = st % NSTAGE;
+        for (int p = 0; p < DEPTH; p++) load(p, p);
+        for (int stu = 0; stu < nst; stu += SLOTS) {
 #pragma unroll
-                for (int i = 0; i < NR; i++) load_raw<KIND>(a, wb, wrow0, t + 32 * UNPACK_WARPS * i, st0 + st + DEPTH, st + DEPTH < nst, raw[DEPTH][i]);
+            for (int u = 0; u < SLOTS; u++) {
+                const int st = stu + u, s = st % NSTAGE;
+                if (st >= nst) break;
+                load((u + DEPTH) % SLOTS, st + DEPTH);
                 if (st >= NSTAGE) mbar_wait(empty(s), ((st / NSTAGE) - 1) & 1, a.err, 20);
 #pragma unroll
-                for (int i = 0; i < NR; i++) store_raw<KIND>(raw[0][i], t + 32 * UNPACK_WARPS * i, smem + s * S::STAGE);
+                for (int i = 0; i < NR; i++) {
+                    const int r = t + 32 * UNPACK_WARPS * i;
+                    if (KIND != FK_Q8_0) store_raw<KIND>(raw[u][i], r, smem + s * S::STAGE);
+                    const StageScale sc = stage_scales<KIND>(rsc[u][i], 4 * (st0 + st));
+                    float* sdw = (float*)(smem + s * S::STAGE + S::DW) + r;
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        float dw, mw;
+                        run_scale<KIND>(sc, j, r, &dw, &mw);
+                        sdw[j * BM] = dw;
+                        if (KIND == FK_Q4_K) sdw[(4 + j) * BM] = mw;
+                    }
+                }
                 fence_proxy_async();   // generic-proxy writes -> visible to the tensor core's reads
                 __syncwarp();
                 if (lane == 0) mbar_arrive(full_a(s));
                 GTR(3, st, warp == EPI_WARPS && lane == 0);
-#pragma unroll
-                for (int p = 0; p < DEPTH; p++)
-#pragma unroll
-                    for (int i = 0; i < NR; i++) raw[p][i] = raw[p + 1][i];
             }
         }
     } else if (warp == EPI_WARPS + UNPACK_WARPS) {
@@ -455,8 +476,8 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap map_q, const _
                 const uint32_t sa = sbase + s * S::STAGE;
                 mbar_expect_tx(full_b(s), TX);
                 tma_load_2d(sa + S::A_BYTES, &map_q, (st0 + st) * KSTAGE, tok0, full_b(s));
-                tma_load_2d(sa + S::A_BYTES + S::B_BYTES, &map_dx, tok0, 4 * (st0 + st), full_b(s));
-                if (KIND == FK_Q4_K) tma_load_2d(sa + S::A_BYTES + S::B_BYTES + S::DX_BYTES, &map_sx, tok0, 4 * (st0 + st), full_b(s));
+                tma_load_2d(sa + S::DX, &map_dx, tok0, 4 * (st0 + st), full_b(s));
+                if (KIND == FK_Q4_K) tma_load_2d(sa + S::DX + S::DX_BYTES, &map_sx, tok0, 4 * (st0 + st), full_b(s));
                 if (KIND == FK_Q8_0) tma_load_3d(sa, &map_w, (st0 + st) * KSTAGE, wrow0, mat, full_b(s));   // [matrix][row][k]: rows past a matrix's end read as zeros
             }
         }
@@ -467,7 +488,7 @@ gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap map_q, const _
             for (int st = 0; st < nst; st++) {
                 const int s = st % NSTAGE;
                 mbar_wait(full_b(s), (st / NSTAGE) & 1, a.err, 40);
-                if (KIND != FK_Q8_0) mbar_wait(full_a(s), (st / NSTAGE) & 1, a.err, 41);
+                mbar_wait(full_a(s), (st / NSTAGE) & 1, a.err, 41);
                 tc_fence_after();
                 const uint32_t sa = sbase + s * S::STAGE;
                 const uint64_t da = umma_desc(sa), db = umma_desc(sa + S::A_BYTES);
@@ -703,14 +724,14 @@ int launch_by_kind(fk_ctx* ctx, cudaStream_t st, const GemmArgs& a, int kind, co
 //
 //   waves * (runs / split * us_per_run(bn) + (split > 1) * exchange(bn)),   waves = CTAs / (SMs * CTAs per SM)
 //
-// The constants were measured on B200 (us; Q4_K, 3072 x 3072, cold L2; the other kinds are within 15 %): a 128-token tile
-// takes 0.82 a run of 32 K, a 64-token one 0.47, a 32-token one 0.40 alone on its SM and 0.56 beside another; the parts of
-// a split tile take 6 to 9 to meet.  A tile's own time hardly falls with its width -- its warps walk the same chain per
-// run -- so what a short prompt needs is more CTAs, not narrower ones: 3072 x 3072, M = 128 was 24 CTAs and 95 us, and is
-// 96 CTAs and 36 us; 3072 x 8192 Q6_K, M = 77 204 -> 81 us; 512 x 3072, M = 16 93 -> 17 us; 8192 x 3072, M = 512 keeps
-// whole 128-token tiles (167 us; 64-token tiles 185, 32-token ones 200).  Grouped: `tiles` expects half a tile of padding
+// The constants were measured on B200 (us; Q4_K, 3072 x 3072, cold L2; the other kinds are within 20 % below): a 128-token
+// tile takes 0.68 a run of 32 K, a 64-token one 0.47, a 32-token one 0.42 alone on its SM and 0.56 beside another; the parts
+// of a split tile take 6 to 8 to meet.  A tile's own time falls far less than its width -- its warps walk the same chain per
+// run -- so what a short prompt needs is more CTAs, not only narrower ones: 3072 x 3072, M = 128 was 24 CTAs and 95 us, and
+// is 96 CTAs and 32 us; 3072 x 8192 Q6_K, M = 77 204 -> 77 us; 512 x 3072, M = 16 93 -> 17 us; 8192 x 3072, M = 512 keeps
+// whole 128-token tiles (142 us; 64-token tiles 181, 32-token ones 204).  Grouped: `tiles` expects half a tile of padding
 // per expert, which is what 32-token tiles win by (128 experts, 8 of them for each of 77 rows, 768 x 2048 Q4_K: the routed
-// layer takes 486 us against 763 with 64-token tiles and 1226 with 128).
+// layer takes 540 us against 755 with 64-token tiles and 1076 with 128).
 struct GemmPlan { int bn, split; };
 
 GemmPlan gemm_plan(const fk_ctx* ctx, const fk_weight_s* w, int m, bool grouped) {
@@ -724,8 +745,8 @@ GemmPlan gemm_plan(const fk_ctx* ctx, const fk_weight_s* w, int m, bool grouped)
             const double ctas = tiles * row_tiles * split;
             const double sms = split == 8 ? 0.9 * ctx->sm_count : ctx->sm_count;       // clusters of eight do not tile every GPC
             const bool two = bn == 32 && ctas > sms;
-            double us = bn == 128 ? (w->kind == FK_MXFP4 ? 1.03 : 0.82) : bn == 64 ? 0.47 : two ? 0.56 : 0.40;
-            us = us * (4 * ((stages + split - 1) / split)) + (split > 1 ? (bn == 128 ? 9.0 : bn == 64 ? 7.0 : 6.0) : 0.0);
+            double us = bn == 128 ? (w->kind == FK_MXFP4 ? 0.80 : 0.68) : bn == 64 ? 0.47 : two ? 0.56 : 0.42;
+            us = us * (4 * ((stages + split - 1) / split)) + (split > 1 ? (bn == 128 ? 8.0 : bn == 64 ? 7.0 : 6.0) : 0.0);
             const double waves = ctas / (two ? 2.0 * sms : sms);
             us *= waves > 4.0 ? waves + 0.25 : ceil(waves);
             if (us < best_us) { best_us = us; best = {bn, split}; }
