@@ -148,6 +148,7 @@ int fk_gemv_bf16_launch(fk_ctx* ctx, cudaStream_t st, fk_weight w, int mat, cons
                         const float* norm_w, float norm_eps, const float* bias, int accumulate);
 int fk_gemv_q5k_launch(fk_ctx* ctx, cudaStream_t st, fk_weight w, int mat, const float* x_dev, int batch, float* y_dev, int32_t* isums_dev);
 // `map` points at a CUtensorMap (128 bytes, 64-byte aligned): [outer][inner] 32-bit words, no swizzle
+int fk_make_map_3d(void* map, void* base, uint32_t inner, uint64_t n1, uint64_t stride1, uint64_t n2, uint32_t b0, uint32_t b1, uint32_t b2, int swizzle);
 int fk_make_map_2d(void* map, int dtype, void* base, uint64_t inner, uint64_t outer, uint32_t box_inner, uint32_t box_outer, int swizzle);
 int fk_make_map_u32(void* map, void* base, uint64_t inner_words, uint64_t outer, uint32_t box_inner, uint32_t box_outer);
 

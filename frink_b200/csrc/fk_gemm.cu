@@ -10,7 +10,7 @@
 // is drained from tensor memory after every K = 32 step and scaled on the CUDA
 // cores; that rescale, not the tensor pipe, bounds this kernel.  Accumulators change hands in groups (half of tensor
 // memory at a time), not run by run, and the launch overlaps the quantizer in front of it (programmatic serialization):
-// with the weight scales decoded by the unpack warps, 8192 x 3072, M = 512 went from 185 to 142 us.
+// with the weight scales decoded by the unpack warps, 8192 x 3072 Q4_K, M = 512 went from 185 to 135 us.
 //
 // One CTA = 128 weight rows x BN tokens (128, 64 or 32; gemm_plan), warps with fixed roles (Tile<BN>):
 //   epilogue    TMEM -> registers (tcgen05.ld), f32 rescale, store
@@ -850,6 +850,23 @@ int fk_make_map_2d(void* map, int dtype, void* base, uint64_t inner, uint64_t ou
     static const int es[4] = {1, 2, 4, 4};
     static const CUtensorMapSwizzle sw[4] = {CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_SWIZZLE_128B};
     return make_map((CUtensorMap*)map, dt[dtype], es[dtype], base, inner, outer, box_inner, box_outer, sw[swizzle]);
+}
+
+// Bytes as a [n2][n1][inner] tensor whose n1 rows lie stride1 bytes apart and whose n2 pieces of a row follow one another
+// (inner bytes apart); box [b2][b1][b0], swizzle as above.
+int fk_make_map_3d(void* map, void* base, uint32_t inner, uint64_t n1, uint64_t stride1, uint64_t n2, uint32_t b0, uint32_t b1, uint32_t b2, int swizzle) {
+    static const CUtensorMapSwizzle sw[4] = {CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_SWIZZLE_128B};
+    EncodeTiledFn fn = encode_fn();
+    if (!fn) return fk_fail(FK_DRIVER_INIT, "the driver does not export cuTensorMapEncodeTiled");
+    cuuint64_t dims[3] = {inner, n1, n2};
+    cuuint64_t strides[2] = {stride1, inner};
+    cuuint32_t box[3] = {b0, b1, b2};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = fn((CUtensorMap*)map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw[swizzle],
+                    CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fk_fail(FK_LAUNCH, "cuTensorMapEncodeTiled failed (%d) for a [%llu][%llu][%u] tensor", (int)r, (unsigned long long)n2,
+                                          (unsigned long long)n1, inner);
+    return FK_OK;
 }
 
 // A [outer][inner] tensor of 32-bit words, unswizzled, for the other kernel files.

@@ -97,7 +97,9 @@ struct GemvArgs {
     int m_chunk_units;     // units of K a stage covers
     int m_xs;              // bytes between batch rows of the quantized activations
     int m_sd_off, m_red_off;
-    int m_srs[4], m_spo[4];   // stage layout: bytes between rows of plane p, offset of plane p
+    int m_p0_bytes, m_rest_bytes;   // a stage's plane 0, its other planes
+    int m_spo[4];             // offset of planes 1.. inside the rest
+    int m_d_pitch;            // Q6_K: bytes between rows of the super-scales
 };
 
 // ------------------------------------------------------------------ PTX glue
@@ -1037,14 +1039,8 @@ __global__ void __launch_bounds__(Q4_MAX_THREADS, 2) gemv_q4k_kernel(const GemvA
 // (g = lane / 4, t = lane % 4), scales them per run in f32 like the dp4a form,
 // and nothing crosses lanes.  The exact int32 dots per run are the same numbers.
 constexpr int MM_ROWS = 16;
-template <int KIND> struct MGeo;
-template <> struct MGeo<FK_Q4_K> { static constexpr int UNIT = 256, PLANES = 1, PB0 = 144, PB1 = 0, PB2 = 0; };
-template <> struct MGeo<FK_Q8_0> { static constexpr int UNIT = 256, PLANES = 2, PB0 = 256, PB1 = 16, PB2 = 0; };
-template <> struct MGeo<FK_Q6_K> { static constexpr int UNIT = 256, PLANES = 4, PB0 = 128, PB1 = 64, PB2 = 16; };
-template <> struct MGeo<FK_MXFP4> { static constexpr int UNIT = 512, PLANES = 2, PB0 = 256, PB1 = 16, PB2 = 0; };
-template <int KIND> __host__ __device__ constexpr int unit_bytes(int p) {
-    return p == 0 ? MGeo<KIND>::PB0 : (p == 1 ? MGeo<KIND>::PB1 : (p == 2 ? MGeo<KIND>::PB2 : 0));
-}
+constexpr int MMA_ALIGN = 1024;   // the 128-byte swizzle's atom
+template <int KIND> struct MGeo { static constexpr int UNIT = KIND == FK_MXFP4 ? 512 : 256; };   // weights of a unit of K
 
 __device__ __forceinline__ uint32_t lds32(uint32_t addr) {
     uint32_t v;
@@ -1063,13 +1059,18 @@ __device__ __forceinline__ uint32_t q6_signed(uint32_t v) {
     return r | (neg << 1) | (neg << 2);
 }
 
-// One stage (units cu0..cu1 of K) of the warp's 16 rows against the batch.
+// One stage (units cu0..cu1 of K) of the warp's 16 rows against the batch.  `stage` is its plane 0, `rest` its other planes.
+// Plane 0 of Q6_K, Q8_0 and MXFP4 stands as [128-byte piece of K][16 rows][128 bytes] in the 128-byte swizzle (16-byte chunk
+// c of row r at chunk c ^ (r & 7)), Q6_K's high bits as [unit][16 rows][64 bytes] in the 64-byte one (c ^ ((r >> 1) & 3)), so
+// the eight rows of a fragment load fall on different banks; scale planes as [16 rows][units of the chunk].
 template <int KIND>
-__device__ __forceinline__ void mma_eat(const GemvArgs& a, uint32_t stage, int cu0, int cu1, uint32_t xrow, const float* sdT, const float* ssT,
-                                        int nb32, int lane, float (&acc)[4]) {
+__device__ __forceinline__ void mma_eat(const GemvArgs& a, uint32_t stage, uint32_t rest, int cu0, int cu1, uint32_t xrow, const float* sdT,
+                                        const float* ssT, int nb32, int lane, float (&acc)[4]) {
     const int g = lane >> 2, t = lane & 3;
-    const uint32_t r0 = stage + a.m_spo[0] + g * a.m_srs[0], r8 = r0 + 8 * a.m_srs[0];
+    const int spitch = a.m_chunk_units * 16;
+    const uint32_t w0 = stage + g * 128 + 4 * t;      // row g of piece 0, row g + 8 is 1024 bytes further on
     if (KIND == FK_Q4_K) {
+        const uint32_t r0 = stage + g * (a.m_chunk_units * 144), r8 = r0 + 8 * (a.m_chunk_units * 144);
         for (int u = cu0; u < cu1; u++) {
             const uint32_t bg = r0 + (u - cu0) * 144, bh = r8 + (u - cu0) * 144;
             const uint4 hg = lds16(bg), hh = lds16(bh);
@@ -1104,16 +1105,17 @@ __device__ __forceinline__ void mma_eat(const GemvArgs& a, uint32_t stage, int c
             }
         }
     } else if (KIND == FK_Q8_0) {
-        const uint32_t s0 = stage + a.m_spo[1] + g * a.m_srs[1], s8 = s0 + 8 * a.m_srs[1];
+        const uint32_t s0 = rest + a.m_spo[1] + g * spitch, s8 = s0 + 8 * spitch;
         for (int u = cu0; u < cu1; u++) {
 #pragma unroll
             for (int r = 0; r < 8; r++) {
                 const int run = u * 8 + r;
                 if (run >= nb32) break;
-                const uint32_t o = ((u - cu0) * 8 + r) * 32 + 4 * t;
+                const uint32_t piece = w0 + ((u - cu0) * 2 + (r >> 2)) * 2048;
+                const uint32_t oa = piece + (((r & 3) * 2) ^ g) * 16, ob = piece + (((r & 3) * 2 + 1) ^ g) * 16;
                 const uint32_t xl = xrow + run * 32 + 4 * t;
                 int d4[4];
-                mma_s8(d4, lds32(r0 + o), lds32(r8 + o), lds32(r0 + o + 16), lds32(r8 + o + 16), lds32(xl), lds32(xl + 16));
+                mma_s8(d4, lds32(oa), lds32(oa + 1024), lds32(ob), lds32(ob + 1024), lds32(xl), lds32(xl + 16));
                 const float wg = fk_h2f((uint16_t)lds_u16(s0 + ((u - cu0) * 8 + r) * 2)), wh = fk_h2f((uint16_t)lds_u16(s8 + ((u - cu0) * 8 + r) * 2));
                 const float2 dx = *(const float2*)(sdT + run * 8 + 2 * t);
                 acc[0] += wg * dx.x * i2f(d4[0]);
@@ -1123,14 +1125,14 @@ __device__ __forceinline__ void mma_eat(const GemvArgs& a, uint32_t stage, int c
             }
         }
     } else if (KIND == FK_MXFP4) {
-        const uint32_t s0 = stage + a.m_spo[1] + g * a.m_srs[1], s8 = s0 + 8 * a.m_srs[1];
+        const uint32_t s0 = rest + a.m_spo[1] + g * spitch, s8 = s0 + 8 * spitch;
         for (int u = cu0; u < cu1; u++) {
 #pragma unroll 4
             for (int r = 0; r < 16; r++) {
                 const int run = u * 16 + r;
                 if (run >= nb32) break;
-                const uint32_t o = ((u - cu0) * 16 + r) * 16 + 4 * t;
-                const uint32_t wg = lds32(r0 + o), wh = lds32(r8 + o);
+                const uint32_t o = w0 + ((u - cu0) * 2 + (r >> 3)) * 2048 + ((r & 7) ^ g) * 16;
+                const uint32_t wg = lds32(o), wh = lds32(o + 1024);
                 // code byte i holds elements i and i + 16; the activations of a run are stored in that (i, i + 16) order
                 const uint32_t xl = xrow + run * 32 + 8 * t;
                 int d4[4];
@@ -1144,22 +1146,22 @@ __device__ __forceinline__ void mma_eat(const GemvArgs& a, uint32_t stage, int c
             }
         }
     } else {   // FK_Q6_K
-        const uint32_t h0 = stage + a.m_spo[1] + g * a.m_srs[1], h8 = h0 + 8 * a.m_srs[1];
-        const uint32_t c0 = stage + a.m_spo[2] + g * a.m_srs[2], c8 = c0 + 8 * a.m_srs[2];
-        const uint32_t d0 = stage + a.m_spo[3] + g * a.m_srs[3], d8 = d0 + 8 * a.m_srs[3];
+        const uint32_t h0 = rest + a.m_spo[1] + g * 64 + 4 * t;            // row g + 8 is 512 bytes further on
+        const uint32_t c0 = rest + a.m_spo[2] + g * spitch, c8 = c0 + 8 * spitch;
+        const uint32_t d0 = rest + a.m_spo[3] + g * a.m_d_pitch, d8 = d0 + 8 * a.m_d_pitch;
         for (int u = cu0; u < cu1; u++) {
             const float dg = fk_h2f((uint16_t)lds_u16(d0 + u * 2)), dh = fk_h2f((uint16_t)lds_u16(d8 + u * 2));   // the whole row's super-scales are staged
             const uint4 scg = lds16(c0 + (u - cu0) * 16), sch = lds16(c8 + (u - cu0) * 16);
             const uint32_t sgw[4] = {scg.x, scg.y, scg.z, scg.w}, shw[4] = {sch.x, sch.y, sch.z, sch.w};
 #pragma unroll
             for (int hf = 0; hf < 2; hf++) {
-                const uint32_t qh_o = (u - cu0) * 64 + 32 * hf + 4 * t;
-                const uint32_t hg0 = lds32(h0 + qh_o), hg1 = lds32(h0 + qh_o + 16), hh0 = lds32(h8 + qh_o), hh1 = lds32(h8 + qh_o + 16);
+                const uint32_t qa = h0 + (u - cu0) * 1024 + ((2 * hf) ^ ((g >> 1) & 3)) * 16, qb = h0 + (u - cu0) * 1024 + ((2 * hf + 1) ^ ((g >> 1) & 3)) * 16;
+                const uint32_t hg0 = lds32(qa), hg1 = lds32(qb), hh0 = lds32(qa + 512), hh1 = lds32(qb + 512);
 #pragma unroll
                 for (int e = 0; e < 4; e++) {      // elements 128 hf + 32 e ..: ql bytes 64 hf + 32 (e & 1) + l, nibble e >> 1, qh bits 2e
-                    const uint32_t ql_o = (u - cu0) * 128 + 64 * hf + 32 * (e & 1) + 4 * t;
+                    const uint32_t la = w0 + (u - cu0) * 2048 + ((4 * hf + 2 * (e & 1)) ^ g) * 16, lb = w0 + (u - cu0) * 2048 + ((4 * hf + 2 * (e & 1) + 1) ^ g) * 16;
                     const int sh = 4 * (e >> 1);
-                    const uint32_t lg0 = lds32(r0 + ql_o), lg1 = lds32(r0 + ql_o + 16), lh0 = lds32(r8 + ql_o), lh1 = lds32(r8 + ql_o + 16);
+                    const uint32_t lg0 = lds32(la), lg1 = lds32(lb), lh0 = lds32(la + 1024), lh1 = lds32(lb + 1024);
                     const uint32_t ag0 = q6_signed(((lg0 >> sh) & 0x0F0F0F0Fu) | (((hg0 >> (2 * e)) & 0x03030303u) << 4));
                     const uint32_t ag1 = q6_signed(((lg1 >> sh) & 0x0F0F0F0Fu) | (((hg1 >> (2 * e)) & 0x03030303u) << 4));
                     const uint32_t ah0 = q6_signed(((lh0 >> sh) & 0x0F0F0F0Fu) | (((hh0 >> (2 * e)) & 0x03030303u) << 4));
@@ -1286,10 +1288,14 @@ __global__ void __launch_bounds__(IMG_THREADS) act_image_kernel(const GemvArgs a
     }
 }
 
+// The planes of a weight matrix as tensors (Q4_K: one).
+struct WeightMaps { CUtensorMap m[4]; };
+
 template <int KIND>
 __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_mma_kernel(const GemvArgs a, const uint8_t* __restrict__ img,
-                                                                   const __grid_constant__ CUtensorMap wmap) {
-    extern __shared__ __align__(128) uint8_t smem[];
+                                                                   const __grid_constant__ WeightMaps wmaps) {
+    extern __shared__ __align__(128) uint8_t smem_raw[];
+    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + MMA_ALIGN - 1) & ~(uintptr_t)(MMA_ALIGN - 1));
     TR(0, threadIdx.x == 0);
     const int cols = a.cols, rows = a.rows, nb32 = cols >> 5, batch = a.batch;
     const int xs = a.m_xs;
@@ -1298,20 +1304,21 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_mma_kernel(const GemvArg
     float* ssT = sdT + nb32 * 8;                        // Q4_K: [nb32][8] scale * run sum
     float4* red = (float4*)(smem + a.m_red_off);        // [2][warps][32] partial sums of the K parts
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint8_t* wb = a.w + (size_t)a.mat * a.mat_stride;
     float* y = a.y;
 
     const uint32_t sbase = smem_u32(smem);
-    const uint32_t ring = sbase + a.act_bytes + warp * (a.nstages * a.stage_bytes);
-    const uint32_t bars = sbase + a.act_bytes + GEMV_WARPS * (a.nstages * a.stage_bytes) + warp * (MAX_STAGES * 8);
-    const uint32_t xbar = sbase + a.act_bytes + GEMV_WARPS * (a.nstages * a.stage_bytes) + GEMV_WARPS * (MAX_STAGES * 8);
+    // plane 0 of every warp's stages, then their other planes: whole swizzle atoms follow one another without padding
+    const uint32_t ring = sbase + a.act_bytes + warp * (a.nstages * a.m_p0_bytes);
+    const uint32_t rest0 = sbase + a.act_bytes + GEMV_WARPS * (a.nstages * a.m_p0_bytes), ring_rest = rest0 + warp * (a.nstages * a.m_rest_bytes);
+    const uint32_t bars = rest0 + GEMV_WARPS * (a.nstages * a.m_rest_bytes) + warp * (MAX_STAGES * 8);
+    const uint32_t xbar = rest0 + GEMV_WARPS * (a.nstages * a.m_rest_bytes) + GEMV_WARPS * (MAX_STAGES * 8);
     if (lane == 0) {
         for (int s = 0; s < a.nstages; s++) mbar_init(bars + 8 * s, 1);
         if (warp == 0) mbar_init(xbar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    constexpr int UNIT = MGeo<KIND>::UNIT, P = MGeo<KIND>::PLANES;
+    constexpr int UNIT = MGeo<KIND>::UNIT;
     const int KS = a.m_ks, gi = warp / KS, kp = warp % KS, GPR = GEMV_WARPS / KS;
     const int ngroups = (rows + MM_ROWS - 1) / MM_ROWS;
     const int units = (cols + UNIT - 1) / UNIT;
@@ -1321,63 +1328,37 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_mma_kernel(const GemvArg
     const int nrounds = first < ngroups ? (ngroups - first + gstride - 1) / gstride : 0;
     const int njobs = nrounds * nch;
 
-    // ---- filling a stage: up to two (row, plane) pieces per lane
-    constexpr int NPIECE = (MM_ROWS * P + 31) / 32;
-    uint32_t f_dst[NPIECE], f_ub[NPIECE], f_pstride[NPIECE];
-    const uint8_t* f_src[NPIECE];
-    int f_r[NPIECE];
-    bool f_whole[NPIECE];
-#pragma unroll
-    for (int i = 0; i < NPIECE; i++) {
-        const int c = lane + 32 * i, r = c / P, p = c % P;
-        f_r[i] = c < MM_ROWS * P ? r : -1;
-        f_whole[i] = KIND == FK_Q6_K && p == 3;
-        const size_t poff = p == 0 ? a.plane_off[0] : p == 1 ? a.plane_off[1] : p == 2 ? a.plane_off[2] : a.plane_off[3];
-        f_pstride[i] = (uint32_t)(p == 0 ? a.plane_stride[0] : p == 1 ? a.plane_stride[1] : p == 2 ? a.plane_stride[2] : a.plane_stride[3]);
-        f_ub[i] = (uint32_t)unit_bytes<KIND>(p);
-        const int srs = p == 0 ? a.m_srs[0] : p == 1 ? a.m_srs[1] : p == 2 ? a.m_srs[2] : a.m_srs[3];
-        const int spo = p == 0 ? a.m_spo[0] : p == 1 ? a.m_spo[1] : p == 2 ? a.m_spo[2] : a.m_spo[3];
-        f_dst[i] = (uint32_t)(spo + r * srs);
-        f_src[i] = wb + poff + (size_t)r * f_pstride[i];
-    }
+    // ---- filling a stage: the 16 rows x chunk of units as ONE tiled copy per plane; a box always has the full size (rows
+    // or pieces past the end arrive as zeros).  One bulk copy per row and plane made 64 copies of 16 to 128 bytes out of a
+    // Q6_K unit, and the copy engine's rate of requests bounded the kernel: 12 matrices of 8192x3072 in Q6_K at batch 8
+    // 243 -> 151 us (1.6 TB/s; what is left is the image's latency and the dot products' instructions), Qwen3-MoE's layers
+    // for eight sequences (Q8_0) 31.3 -> 21.5 ms for 48 tokens.
     int f_stage = 0, f_ch = 0, f_group = first;
+    auto copy2 = [&](uint32_t dst, const CUtensorMap* m, int x, int y0, uint32_t bar) {
+        asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                     ::"r"(dst), "l"(m), "r"(x), "r"(y0), "r"(bar) : "memory");
+    };
+    auto copy3 = [&](uint32_t dst, const CUtensorMap* m, int y0, int z, uint32_t bar) {
+        asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+                     ::"r"(dst), "l"(m), "r"(0), "r"(y0), "r"(z), "r"(bar) : "memory");
+    };
     auto fill = [&]() {
-        const uint32_t stage = ring + f_stage * a.stage_bytes, bar = bars + 8 * f_stage;
-        const int cu0 = u0 + f_ch * a.m_chunk_units, cu1 = min(u1, cu0 + a.m_chunk_units);
-        if (KIND == FK_Q4_K) {
-            // the 16 rows x chunk of blocks as ONE tiled copy (the matrix is a [rows][row words] tensor);
-            // the box always has the full size: rows or blocks past the end arrive as zeros
-            if (lane == 0) {
-                mbar_expect_tx(bar, (uint32_t)a.stage_bytes);
-                asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                             ::"r"(stage), "l"(&wmap), "r"(cu0 * 36), "r"(f_group * MM_ROWS), "r"(bar) : "memory");
-            }
-            if (++f_stage == a.nstages) f_stage = 0;
-            if (++f_ch == nch) { f_ch = 0; f_group += gstride; }
-            return;
-        }
-        uint32_t off[NPIECE], bytes[NPIECE], mine = 0;
-#pragma unroll
-        for (int i = 0; i < NPIECE; i++) {
-            off[i] = 0;
-            bytes[i] = 0;
-            if (f_r[i] >= 0 && f_group * MM_ROWS + f_r[i] < rows) {
-                if (f_whole[i]) {
-                    bytes[i] = f_pstride[i];
-                } else {
-                    off[i] = (uint32_t)cu0 * f_ub[i];
-                    bytes[i] = (uint32_t)(cu1 - cu0) * f_ub[i];
-                    if (off[i] + bytes[i] > f_pstride[i]) bytes[i] = f_pstride[i] - off[i];   // the ragged end of a row (strides are padded to 16)
-                }
-                mine += bytes[i];
+        if (lane == 0) {
+            const uint32_t p0 = ring + f_stage * a.m_p0_bytes, rest = ring_rest + f_stage * a.m_rest_bytes, bar = bars + 8 * f_stage;
+            const int cu0 = u0 + f_ch * a.m_chunk_units, row0 = f_group * MM_ROWS;
+            mbar_expect_tx(bar, (uint32_t)a.stage_bytes);
+            if (KIND == FK_Q4_K) {
+                copy2(p0, &wmaps.m[0], cu0 * 36, row0, bar);
+            } else if (KIND == FK_Q6_K) {
+                copy3(p0, &wmaps.m[0], row0, cu0, bar);
+                copy3(rest + a.m_spo[1], &wmaps.m[1], row0, cu0, bar);
+                copy2(rest + a.m_spo[2], &wmaps.m[2], cu0 * 16, row0, bar);
+                copy2(rest + a.m_spo[3], &wmaps.m[3], 0, row0, bar);          // the whole row's super-scales
+            } else {
+                copy3(p0, &wmaps.m[0], row0, 2 * cu0, bar);
+                copy2(rest + a.m_spo[1], &wmaps.m[1], cu0 * 16, row0, bar);
             }
         }
-        const uint32_t total = __reduce_add_sync(0xffffffffu, mine);
-        if (lane == 0) mbar_expect_tx(bar, total);
-        __syncwarp();
-#pragma unroll
-        for (int i = 0; i < NPIECE; i++)
-            if (bytes[i]) bulk_g2s(stage + f_dst[i], f_src[i] + (size_t)f_group * MM_ROWS * f_pstride[i] + off[i], bytes[i], bar);
         if (++f_stage == a.nstages) f_stage = 0;
         if (++f_ch == nch) { f_ch = 0; f_group += gstride; }
     };
@@ -1405,7 +1386,7 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_mma_kernel(const GemvArg
             mbar_wait(bars + 8 * s, phase, a.err);
             TR(4, threadIdx.x == 0 && round == 0 && ch == 0);
             const int cu0 = u0 + ch * a.m_chunk_units, cu1 = min(u1, cu0 + a.m_chunk_units);
-            mma_eat<KIND>(a, ring + s * a.stage_bytes, cu0, cu1, xrow, sdT, ssT, nb32, lane, acc);
+            mma_eat<KIND>(a, ring + s * a.m_p0_bytes, ring_rest + s * a.m_rest_bytes, cu0, cu1, xrow, sdT, ssT, nb32, lane, acc);
             __syncwarp();
             TR(5, threadIdx.x == 0 && round == 0 && ch == 0);
             if ((round * nch + ch) + a.nstages < njobs) fill();
@@ -1604,7 +1585,7 @@ int launch_q4k(fk_ctx* ctx, cudaStream_t st, GemvArgs a, const fk_weight_s* w, i
 // stage of one unit does not fit, and the caller falls back to the dp4a form.
 template <int KIND>
 int launch_mma(fk_ctx* ctx, cudaStream_t st, GemvArgs a, const fk_weight_s* w, bool* fits) {
-    constexpr int UNIT = MGeo<KIND>::UNIT, P = MGeo<KIND>::PLANES;
+    constexpr int UNIT = MGeo<KIND>::UNIT;
     *fits = false;
     const int units = (a.cols + UNIT - 1) / UNIT, nb32 = a.cols / 32;
     const int ngroups = (a.rows + MM_ROWS - 1) / MM_ROWS;
@@ -1619,43 +1600,50 @@ int launch_mma(fk_ctx* ctx, cudaStream_t st, GemvArgs a, const fk_weight_s* w, b
     act += (size_t)nb32 * 32 * (KIND == FK_Q4_K ? 2 : 1);
     act = (act + 15) & ~(size_t)15;
     a.m_red_off = (int)act;
-    act += 2 * GEMV_WARPS * 32 * 16;
-    act = (act + 127) & ~(size_t)127;
+    if (ks > 1) act += 2 * GEMV_WARPS * 32 * 16;
+    act = (act + MMA_ALIGN - 1) & ~(size_t)(MMA_ALIGN - 1);
     const int bars = GEMV_WARPS * MAX_STAGES * 8 + 16;   // + the barrier of the activation image
-    const int ring_budget = ((int)SMEM_BUDGET - (int)act - bars) / GEMV_WARPS;
-    auto layout = [&](int cu, int* srs, int* spo) {
-        int off = 0;
-        for (int p = 0; p < P; p++) {
-            int b = (KIND == FK_Q6_K && p == 3) ? (int)w->plane_stride[3] : cu * unit_bytes<KIND>(p);
-            b = (b + 15) & ~15;
-            // rows 16 mod 32 bytes apart: the eight rows of a fragment load hit different banks
-            // (Q4_K arrives as a dense tile: an odd number of 144-byte blocks per chunk does it)
-            if ((b & 31) == 0 && KIND != FK_Q4_K) b += 16;
-            srs[p] = b;
-            spo[p] = off;
-            off += MM_ROWS * b;
+    // MMA_ALIGN in front (the swizzled planes start on whole atoms) and MMA_ALIGN of rounding come on top of the budget,
+    // 227 KB in all: the widest rows still fit
+    const int ring_budget = ((int)SMEM_BUDGET + MMA_ALIGN - (int)act - bars) / GEMV_WARPS;
+    if (KIND == FK_Q6_K && w->plane_stride[3] > 256) return FK_UNSUPPORTED;      // a row's super-scales are one box row of at most 256 bytes
+    a.m_d_pitch = (int)w->plane_stride[3];
+    // bytes of a stage of cu units: plane 0, then the other planes (512-byte steps keep the swizzled ones aligned)
+    auto layout = [&](int cu, GemvArgs& g) {
+        g.m_p0_bytes = KIND == FK_Q4_K ? cu * 144 * MM_ROWS : cu * (KIND == FK_Q6_K ? 1 : 2) * 2048;
+        int rest = 0;
+        g.m_spo[1] = g.m_spo[2] = g.m_spo[3] = 0;
+        if (KIND == FK_Q6_K) {
+            g.m_spo[2] = rest += cu * 1024;
+            g.m_spo[3] = rest += cu * 16 * MM_ROWS;
+            rest += MM_ROWS * g.m_d_pitch;
+        } else if (KIND != FK_Q4_K) {
+            rest += cu * 16 * MM_ROWS;
         }
-        return off;
+        g.stage_bytes = g.m_p0_bytes + rest;
+        g.m_rest_bytes = (rest + 511) & ~511;
+        return g.m_p0_bytes + g.m_rest_bytes;
     };
-    int srs[4] = {0, 0, 0, 0}, spo[4] = {0, 0, 0, 0};
     int cu = a.m_kpart_units;
     if (KIND == FK_Q4_K) {
         if (cu > 7) cu = 7;                 // a tile is at most 256 words wide
+        // rows an odd number of 144-byte blocks apart: the eight rows of a fragment load hit different banks
         if ((cu & 1) == 0) cu--;
-        while (cu > 1 && 2 * layout(cu, srs, spo) > ring_budget) cu -= 2;
+        while (cu > 1 && 2 * layout(cu, a) > ring_budget) cu -= 2;
     } else {
-        while (cu > 1 && 2 * layout(cu, srs, spo) > ring_budget) cu--;
+        if (cu > 16) cu = 16;               // a scale tile is at most 256 bytes wide
+        while (cu > 1 && 2 * layout(cu, a) > ring_budget) cu--;
+        const int nch = (a.m_kpart_units + cu - 1) / cu;      // boxes have one size: an even cut leaves the last one full
+        cu = (a.m_kpart_units + nch - 1) / nch;
     }
-    const int stage = layout(cu, srs, spo);
+    const int stage = layout(cu, a);
     if (ring_budget <= 0 || stage > ring_budget) return FK_UNSUPPORTED;
     *fits = true;
     a.m_chunk_units = cu;
-    for (int p = 0; p < 4; p++) { a.m_srs[p] = srs[p]; a.m_spo[p] = spo[p]; }
-    a.stage_bytes = stage;
     a.nstages = ring_budget / stage;
     if (a.nstages > MAX_STAGES) a.nstages = MAX_STAGES;
     a.act_bytes = (int)act;
-    const size_t smem = act + (size_t)GEMV_WARPS * a.nstages * a.stage_bytes + bars;
+    const size_t smem = MMA_ALIGN + act + (size_t)GEMV_WARPS * a.nstages * stage + bars;
     auto kern = gemv_mma_kernel<KIND>;
     {
         // raise the kernel's dynamic shared-memory limit only when this launch needs more than any
@@ -1688,15 +1676,29 @@ int launch_mma(fk_ctx* ctx, cudaStream_t st, GemvArgs a, const fk_weight_s* w, b
     icfg.gridDim = dim3((unsigned)a.batch);
     icfg.blockDim = dim3(IMG_THREADS);
     icfg.dynamicSmemBytes = 0;
-    alignas(64) CUtensorMap wmap;
-    memset(&wmap, 0, sizeof(wmap));
+    alignas(64) WeightMaps maps;
+    memset(&maps, 0, sizeof(maps));
+    auto plane = [&](int p) { return (void*)(w->dev + (size_t)a.mat * w->mat_stride + w->plane_off[p]); };
+    const uint64_t rows = (uint64_t)a.rows;
+    int rcm;
     if (KIND == FK_Q4_K) {
-        const int rcm = fk_make_map_u32(&wmap, (void*)(w->dev + (size_t)a.mat * w->mat_stride + w->plane_off[0]), w->plane_stride[0] / 4,
-                                        (uint64_t)a.rows, (uint32_t)(36 * cu), MM_ROWS);
-        if (rcm != FK_OK) return rcm;
+        rcm = fk_make_map_u32(&maps.m[0], plane(0), w->plane_stride[0] / 4, rows, (uint32_t)(36 * cu), MM_ROWS);
+    } else {
+        // plane 0 (and Q6_K's plane 1) as [piece of K][row][piece bytes]: pieces of a row are contiguous, so a ragged last
+        // piece reads into the next row (the last row: into the plane's 256 bytes of slack); nothing uses those bytes
+        const uint32_t pieces = KIND == FK_Q6_K ? 1 : 2;      // 128-byte pieces of a unit
+        rcm = fk_make_map_3d(&maps.m[0], plane(0), 128, rows, w->plane_stride[0], (w->plane_stride[0] + 127) / 128, 128, MM_ROWS, pieces * cu, 3);
+        if (rcm == FK_OK && KIND == FK_Q6_K) {
+            rcm = fk_make_map_3d(&maps.m[1], plane(1), 64, rows, w->plane_stride[1], w->plane_stride[1] / 64, 64, MM_ROWS, cu, 2);
+            if (rcm == FK_OK) rcm = fk_make_map_2d(&maps.m[2], 0, plane(2), w->plane_stride[2], rows, 16 * cu, MM_ROWS, 0);
+            if (rcm == FK_OK) rcm = fk_make_map_2d(&maps.m[3], 0, plane(3), w->plane_stride[3], rows, (uint32_t)w->plane_stride[3], MM_ROWS, 0);
+        } else if (rcm == FK_OK) {
+            rcm = fk_make_map_2d(&maps.m[1], 0, plane(1), w->plane_stride[1], rows, 16 * cu, MM_ROWS, 0);
+        }
     }
+    if (rcm != FK_OK) return rcm;
     FK_CUDA(cudaLaunchKernelEx(&icfg, act_image_kernel<KIND>, a, ctx->scratch), FK_LAUNCH);
-    FK_CUDA(cudaLaunchKernelEx(&cfg, kern, a, img, wmap), FK_LAUNCH);
+    FK_CUDA(cudaLaunchKernelEx(&cfg, kern, a, img, maps), FK_LAUNCH);
     ctx->launches += 2;
     return FK_OK;
 }
