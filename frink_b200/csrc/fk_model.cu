@@ -442,22 +442,27 @@ attn_kernel(const float* __restrict__ q, int q_ld, const float* __restrict__ kbu
     if (threadIdx.x == 0) cnt[r * n_heads + h] = 0;
 }
 
-// ---- the same attention for a prefill batch: a block takes 32 consecutive query rows
-// of one head, 8 warps x 4 rows; K and V tiles of 32 keys are staged once in shared
-// memory (K rows padded by 4 floats so lanes scoring different keys hit different
-// banks) and shared by the block's 32 rows.
-constexpr int PF_ROWS = 32, PF_WARPS = 8, PF_RPW = PF_ROWS / PF_WARPS;
+// ---- the same attention for a prefill batch: a block takes 8 * RPW consecutive query rows of one head, 8 warps x RPW
+// rows; K and V tiles of 32 keys are staged once in shared memory (K rows padded by 4 floats so lanes scoring different
+// keys hit different banks) and shared by the block's rows.  Bound by the chain load tile -> stage -> score -> fold of a
+// block, not by arithmetic: the next tile is requested into registers before the current one is scored, and a prompt too
+// short to give every SM two blocks of 32 rows takes blocks of 16 or 8 rows (24 heads of 128: 13.4 -> 9.4 us at 40
+// tokens, 31.6 -> 26.7 at 128, 75.6 -> 64.9 at 256, 167.5 -> 157.3 at 512, where the blocks stay 32 rows high).  A row's own sums run in the
+// same order whatever the block height.
+constexpr int PF_WARPS = 8;
+template <int RPW>
 __global__ void __launch_bounds__(PF_WARPS * 32)
 attn_prefill_kernel(const float* __restrict__ q, int q_ld, const float* __restrict__ kbuf, const float* __restrict__ vbuf, int n_q, int n_heads, int n_kv,
                     int head_dim, const int* __restrict__ pos, float scale, float* __restrict__ out, int cache_rows, int* __restrict__ err,
                     int window, const float* __restrict__ sinks) {
     if (fk_cache_overrun(*pos, n_q, cache_rows, err)) return;
+    constexpr int PF_ROWS = PF_WARPS * RPW;
     extern __shared__ __align__(16) float sm[];
     const int kpad = head_dim + 4;
-    float* sq = sm;                          // [32][head_dim]
+    float* sq = sm;                          // [PF_ROWS][head_dim]
     float* sk = sq + PF_ROWS * head_dim;     // [32][head_dim + 4]
     float* sv = sk + 32 * kpad;              // [32][head_dim]
-    const int r0 = blockIdx.x * PF_ROWS, h = blockIdx.y, kvh = h / (n_heads / n_kv);
+    const int r0 = (gridDim.x - 1 - blockIdx.x) * PF_ROWS, h = blockIdx.y, kvh = h / (n_heads / n_kv);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int p0 = *pos;
     const size_t kv_stride = (size_t)n_kv * head_dim;
@@ -468,38 +473,53 @@ attn_prefill_kernel(const float* __restrict__ q, int q_ld, const float* __restri
         if (r0 + rr < n_q) v = *(const float4*)(q + (size_t)(r0 + rr) * q_ld + (size_t)h * head_dim + 4 * c);
         *(float4*)(sq + rr * head_dim + 4 * c) = v;
     }
-    float m[PF_RPW], s[PF_RPW];
-    float4 acc[PF_RPW];
+    float m[RPW], s[RPW];
+    float4 acc[RPW];
 #pragma unroll
-    for (int i = 0; i < PF_RPW; i++) { m[i] = -INFINITY; s[i] = 0.0f; acc[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f); }
+    for (int i = 0; i < RPW; i++) { m[i] = -INFINITY; s[i] = 0.0f; acc[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f); }
     const bool owns = 4 * lane < head_dim;
     const int last_row = min(n_q, r0 + PF_ROWS) - 1;
     const int n_keys_max = p0 + last_row + 1;
     // with a window, the block's first row sees the oldest key: tiles before it are skipped (32-aligned, so the tiles are
     // the same as without a window)
     const int t_first = window > 0 ? (max(0, p0 + r0 + 1 - window) & ~31) : 0;
+    // a thread's share of a tile (head_dim <= 128: at most four 16-byte pieces of K and of V), requested a tile ahead
+    constexpr int PIECES = 32 * 32 / (PF_WARPS * 32);
+    float4 pk[PIECES], pv[PIECES];
+    auto request = [&](int t0) {
+#pragma unroll
+        for (int u = 0; u < PIECES; u++) {
+            const int i = u * PF_WARPS * 32 + threadIdx.x;
+            pk[u] = pv[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (i < 32 * hd4 && t0 + i / hd4 < n_keys_max) {
+                const size_t at = (size_t)(t0 + i / hd4) * kv_stride + (size_t)kvh * head_dim + 4 * (i % hd4);
+                pk[u] = *(const float4*)(kbuf + at);
+                pv[u] = *(const float4*)(vbuf + at);
+            }
+        }
+    };
+    request(t_first);
     for (int t0 = t_first; t0 < n_keys_max; t0 += 32) {
         __syncthreads();
-        for (int i = threadIdx.x; i < 32 * hd4; i += blockDim.x) {
-            const int kk = i / hd4, c = i % hd4;
-            float4 kv4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), vv4 = kv4;
-            if (t0 + kk < n_keys_max) {
-                kv4 = *(const float4*)(kbuf + (size_t)(t0 + kk) * kv_stride + (size_t)kvh * head_dim + 4 * c);
-                vv4 = *(const float4*)(vbuf + (size_t)(t0 + kk) * kv_stride + (size_t)kvh * head_dim + 4 * c);
+#pragma unroll
+        for (int u = 0; u < PIECES; u++) {
+            const int i = u * PF_WARPS * 32 + threadIdx.x;
+            if (i < 32 * hd4) {
+                *(float4*)(sk + (i / hd4) * kpad + 4 * (i % hd4)) = pk[u];
+                *(float4*)(sv + (i / hd4) * head_dim + 4 * (i % hd4)) = pv[u];
             }
-            *(float4*)(sk + kk * kpad + 4 * c) = kv4;
-            *(float4*)(sv + kk * head_dim + 4 * c) = vv4;
         }
+        if (t0 + 32 < n_keys_max) request(t0 + 32);
         __syncthreads();
         // the warp's rows together: a key's row of K (and of V below) is read once from shared memory for all of them.
         // Every row's own sums run in the same order as if it were alone.
         const int key = t0 + lane;
-        int nk[PF_RPW], lo[PF_RPW];
-        bool act[PF_RPW];
-        float d[PF_RPW], p[PF_RPW];
+        int nk[RPW], lo[RPW];
+        bool act[RPW];
+        float d[RPW], p[RPW];
 #pragma unroll
-        for (int i = 0; i < PF_RPW; i++) {
-            const int r = r0 + warp * PF_RPW + i;
+        for (int i = 0; i < RPW; i++) {
+            const int r = r0 + warp * RPW + i;
             nk[i] = p0 + r + 1;
             lo[i] = window > 0 ? max(0, nk[i] - window) : 0;
             act[i] = r < n_q && t0 < nk[i] && t0 + 32 > lo[i];
@@ -508,15 +528,16 @@ attn_prefill_kernel(const float* __restrict__ q, int q_ld, const float* __restri
         }
         bool any = false;
 #pragma unroll
-        for (int i = 0; i < PF_RPW; i++) any = any || act[i];
+        for (int i = 0; i < RPW; i++) any = any || act[i];
         if (!any) continue;                                  // none of the warp's rows sees this tile
         {
             const float* kr = sk + lane * kpad;
-            const float* qr = sq + warp * PF_RPW * head_dim;
+            const float* qr = sq + warp * RPW * head_dim;
+#pragma unroll 4
             for (int c = 0; c < hd4; c++) {
                 const float4 kv4 = *(const float4*)(kr + 4 * c);
 #pragma unroll
-                for (int i = 0; i < PF_RPW; i++) {
+                for (int i = 0; i < RPW; i++) {
                     const float4 qv = *(const float4*)(qr + i * head_dim + 4 * c);
                     d[i] += kv4.x * qv.x + kv4.y * qv.y + kv4.z * qv.z + kv4.w * qv.w;
                 }
@@ -524,7 +545,7 @@ attn_prefill_kernel(const float* __restrict__ q, int q_ld, const float* __restri
         }
         int cnt = 0;
 #pragma unroll
-        for (int i = 0; i < PF_RPW; i++) {
+        for (int i = 0; i < RPW; i++) {
             if (!act[i]) continue;
             const bool vis = key < nk[i] && key >= lo[i];
             const float sc = vis ? d[i] * scale : -INFINITY;
@@ -540,19 +561,20 @@ attn_prefill_kernel(const float* __restrict__ q, int q_ld, const float* __restri
             m[i] = m_new;
             cnt = max(cnt, min(32, nk[i] - t0));
         }
+#pragma unroll 4
         for (int j = 0; j < cnt; j++) {
             float4 vv = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             if (owns) vv = *(const float4*)(sv + j * head_dim + 4 * lane);
 #pragma unroll
-            for (int i = 0; i < PF_RPW; i++) {
+            for (int i = 0; i < RPW; i++) {
                 const float pj = __shfl_sync(0xffffffffu, p[i], j);
                 acc[i].x += pj * vv.x; acc[i].y += pj * vv.y; acc[i].z += pj * vv.z; acc[i].w += pj * vv.w;
             }
         }
     }
 #pragma unroll
-    for (int i = 0; i < PF_RPW; i++) {
-        const int r = r0 + warp * PF_RPW + i;
+    for (int i = 0; i < RPW; i++) {
+        const int r = r0 + warp * RPW + i;
         if (r < n_q && owns) {
             const float inv = 1.0f / (sinks ? s[i] + expf(sinks[h] - m[i]) : s[i]);
             float* orow = out + ((size_t)r * n_heads + h) * head_dim + 4 * lane;
@@ -737,10 +759,14 @@ FK_EXPORT int fk_attention(fk_ctx* ctx, void* stream, const float* q_dev, int q_
     if (q_ld < n_heads * head_dim || (q_ld & 3) || ((uintptr_t)q_dev & 15)) return fk_fail(FK_INVALID, "attention: query row stride %d", q_ld);
     FkDeviceGuard g(ctx->device);
     if (n_q >= 16) {
-        const size_t smem = (size_t)(PF_ROWS * head_dim + 32 * (head_dim + 4) + 32 * head_dim) * sizeof(float);
-        FK_CUDA(cudaFuncSetAttribute(attn_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), FK_KERNEL);
-        FK_CARVEOUT(attn_prefill_kernel);
-        attn_prefill_kernel<<<dim3((n_q + PF_ROWS - 1) / PF_ROWS, n_heads), PF_WARPS * 32, smem, (cudaStream_t)stream>>>(
+        auto blocks = [&](int rpw) { return (n_q + PF_WARPS * rpw - 1) / (PF_WARPS * rpw) * n_heads; };
+        int rpw = 4;
+        while (rpw > 1 && blocks(rpw) < 2 * ctx->sm_count) rpw >>= 1;
+        auto kern = rpw == 4 ? attn_prefill_kernel<4> : rpw == 2 ? attn_prefill_kernel<2> : attn_prefill_kernel<1>;
+        const size_t smem = (size_t)(PF_WARPS * rpw * head_dim + 32 * (head_dim + 4) + 32 * head_dim) * sizeof(float);
+        FK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), FK_KERNEL);
+        FK_CARVEOUT(kern);
+        kern<<<dim3(blocks(rpw) / n_heads, n_heads), PF_WARPS * 32, smem, (cudaStream_t)stream>>>(
             q_dev, q_ld, k_dev, v_dev, n_q, n_heads, n_kv, head_dim, pos_dev, scale, out_dev, cache_rows, ctx->err_flag, window, sinks_dev);
     } else {
         if (n_q * n_heads > AD_MAX_CNT) return fk_fail(FK_UNSUPPORTED, "attention: %d rows x %d heads", n_q, n_heads);
