@@ -76,7 +76,7 @@ struct GemvArgs {
                            //   launches old), so it may be read -- and the activations prepared -- before the wait on that kernel
     // plan of the Q4_K batch 1..2 kernel (block-owned row ranges)
     int q_lp;              // row pairs a warp tile spans (32, 16 or 8; the rest of the lanes span super-blocks)
-    int q_sc_off, q_part_off, q_ring_off, q_bar_off;
+    int q_sc_off, q_part_off, q_part_ld, q_ring_off, q_bar_off;
 #ifdef FK_TRACE
     int trace_slot;
 #endif
@@ -847,7 +847,7 @@ __global__ void __launch_bounds__(Q4_MAX_THREADS, 2) gemv_q4k_kernel(const GemvA
     const int cols = a.cols, rows = a.rows, nb32 = cols >> 5, nsb = cols >> 8;
     int8_t* sq = (int8_t*)smem;                               // [NB][cols] int8
     float* ssc = (float*)(smem + a.q_sc_off);                  // [NB][nsb][16]: per super-block d[0..7], d * run sum [0..7]
-    float* part = (float*)(smem + a.q_part_off);               // [block rows][nsb][NB]
+    float* part = (float*)(smem + a.q_part_off);               // [block rows][q_part_ld][NB]
     const uint32_t sbase = smem_u32(smem), ring = sbase + a.q_ring_off, bar = sbase + a.q_bar_off;
     const uint8_t* wb = a.w + (size_t)a.mat * a.mat_stride;
     const float* x = a.x;
@@ -882,18 +882,26 @@ __global__ void __launch_bounds__(Q4_MAX_THREADS, 2) gemv_q4k_kernel(const GemvA
     // ---- activations -> q8_1 in shared memory (the rule of fk_q8_1_lane; eight lanes make a run)
     const int c4 = cols >> 2, items = NB * c4;
     constexpr int QU = 1024 / Q4_MAX_THREADS;
-    for (int base = 0; base < items; base += QU * T) {
-        float4 v[QU];
+    // the next pass over x is requested before this one is quantized: with 8192 columns (two passes) the second wait for L2
+    // came on top of the first (with the odd pitch of the partial sums, 3072x8192: 7.1 -> 6.1 us a launch)
+    float4 v[QU], nx[QU];
+    auto request = [&](int base) {
 #pragma unroll
         for (int u = 0; u < QU; u++) {
             const int idx = base + u * T + tid;
-            v[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            nx[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             if (idx < items) {
                 const int b = NB == 1 ? 0 : idx / c4, k4 = idx - b * c4;
                 // x may be written by the kernel this one overlaps with: read it past L1
-                if (b < a.batch) v[u] = __ldcg((const float4*)(x + (size_t)b * a.x_ld) + k4);
+                if (b < a.batch) nx[u] = __ldcg((const float4*)(x + (size_t)b * a.x_ld) + k4);
             }
         }
+    };
+    request(0);
+    for (int base = 0; base < items; base += QU * T) {
+#pragma unroll
+        for (int u = 0; u < QU; u++) v[u] = nx[u];
+        request(base + QU * T);
 #pragma unroll
         for (int u = 0; u < QU; u++) {
             if (base + u * T + warp * 32 >= items) continue;   // nothing for this warp here (the same for all its lanes)
@@ -1013,7 +1021,7 @@ __global__ void __launch_bounds__(Q4_MAX_THREADS, 2) gemv_q4k_kernel(const GemvA
         for (int r = 0; r < 2; r++)
 #pragma unroll
             for (int b = 0; b < NB; b++)
-                if (r == 0 || two) part[((size_t)(2 * pr + r) * nsb + sb) * NB + b] = dd[r] * accS[r][b] - dm[r] * accM[r][b];
+                if (r == 0 || two) part[((2 * pr + r) * a.q_part_ld + sb) * NB + b] = dd[r] * accS[r][b] - dm[r] * accM[r][b];
     }
     __syncthreads();
     TR(5, threadIdx.x == 0);
@@ -1022,7 +1030,7 @@ __global__ void __launch_bounds__(Q4_MAX_THREADS, 2) gemv_q4k_kernel(const GemvA
         const int rr = i / NB, b = i - rr * NB;
         if (b >= a.batch) continue;
         float v = 0.0f;
-        for (int k = 0; k < nsb; k++) v += part[((size_t)rr * nsb + k) * NB + b];
+        for (int k = 0; k < nsb; k++) v += part[(rr * a.q_part_ld + k) * NB + b];
         y[(size_t)b * rows + row_lo + rr] = v;
     }
     TR(6, threadIdx.x == 0);
@@ -1550,9 +1558,12 @@ int launch_q4k(fk_ctx* ctx, cudaStream_t st, GemvArgs a, const fk_weight_s* w, i
         if (rounds < best) { best = rounds; lp = c; }
     }
     a.q_lp = lp;
+    // a row's partial sums an odd number of words from the next row's (nsb = 32: the threads that add them up all met on one
+    // bank), where the few bytes are there
+    a.q_part_ld = fixed + (size_t)ppb * (per_pair + 8 * NB) <= budget ? nsb | 1 : nsb;
     a.q_sc_off = NB * a.cols;
     a.q_part_off = a.q_sc_off + NB * nsb * 64;
-    a.q_ring_off = (int)(((size_t)a.q_part_off + 2 * (size_t)ppb * nsb * NB * 4 + 127) & ~(size_t)127);
+    a.q_ring_off = (int)(((size_t)a.q_part_off + 2 * (size_t)ppb * a.q_part_ld * NB * 4 + 127) & ~(size_t)127);
     a.q_bar_off = a.q_ring_off + (int)((size_t)ppb * (2 * rb + 16));
     const size_t smem = (size_t)a.q_bar_off + 64;
     auto kern = gemv_q4k_kernel<NB, DUMP>;
