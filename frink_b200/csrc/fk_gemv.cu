@@ -1048,7 +1048,11 @@ __global__ void __launch_bounds__(Q4_MAX_THREADS, 2) gemv_q4k_kernel(const GemvA
 // and nothing crosses lanes.  The exact int32 dots per run are the same numbers.
 constexpr int MM_ROWS = 16;
 constexpr int MMA_ALIGN = 1024;   // the 128-byte swizzle's atom
-template <int KIND> struct MGeo { static constexpr int UNIT = KIND == FK_MXFP4 ? 512 : 256; };   // weights of a unit of K
+template <int KIND> struct MGeo {
+    static constexpr int UNIT = KIND == FK_MXFP4 ? 512 : 256;      // weights of a unit of K
+    // Q4_K, Q5_K: one plane of whole super-blocks (scales and mins in front), the others several
+    static constexpr int BLOCK = KIND == FK_Q4_K ? 144 : KIND == FK_Q5_K ? 176 : 0;
+};
 
 __device__ __forceinline__ uint32_t lds32(uint32_t addr) {
     uint32_t v;
@@ -1077,10 +1081,11 @@ __device__ __forceinline__ void mma_eat(const GemvArgs& a, uint32_t stage, uint3
     const int g = lane >> 2, t = lane & 3;
     const int spitch = a.m_chunk_units * 16;
     const uint32_t w0 = stage + g * 128 + 4 * t;      // row g of piece 0, row g + 8 is 1024 bytes further on
-    if (KIND == FK_Q4_K) {
-        const uint32_t r0 = stage + g * (a.m_chunk_units * 144), r8 = r0 + 8 * (a.m_chunk_units * 144);
+    if constexpr (MGeo<KIND>::BLOCK > 0) {
+        constexpr int BB = MGeo<KIND>::BLOCK, QS = BB - 128;      // Q5_K: 32 bytes of fifth bits between the scales and the nibbles
+        const uint32_t r0 = stage + g * (a.m_chunk_units * BB), r8 = r0 + 8 * (a.m_chunk_units * BB);
         for (int u = cu0; u < cu1; u++) {
-            const uint32_t bg = r0 + (u - cu0) * 144, bh = r8 + (u - cu0) * 144;
+            const uint32_t bg = r0 + (u - cu0) * BB, bh = r8 + (u - cu0) * BB;
             const uint4 hg = lds16(bg), hh = lds16(bh);
             // 6-bit scales and mins of the 8 sub-blocks, one per byte: [0..3] and [4..7]
             const uint32_t scg[2] = {hg.y & 0x3F3F3F3Fu, (hg.w & 0x0F0F0F0Fu) | ((hg.y >> 2) & 0x30303030u)};
@@ -1089,16 +1094,24 @@ __device__ __forceinline__ void mma_eat(const GemvArgs& a, uint32_t stage, uint3
             const uint32_t mnh[2] = {hh.z & 0x3F3F3F3Fu, ((hh.w >> 4) & 0x0F0F0F0Fu) | ((hh.z >> 2) & 0x30303030u)};
             const float dg = fk_h2f((uint16_t)(hg.x & 0xFFFF)), ndming = -fk_h2f((uint16_t)(hg.x >> 16));
             const float dh = fk_h2f((uint16_t)(hh.x & 0xFFFF)), ndminh = -fk_h2f((uint16_t)(hh.x >> 16));
+            uint32_t h0 = 0, h1 = 0, h2 = 0, h3 = 0;       // Q5_K: bit i of a byte is the fifth bit of run i
+            if (KIND == FK_Q5_K) {
+                h0 = lds32(bg + 16 + 4 * t); h2 = lds32(bg + 32 + 4 * t);
+                h1 = lds32(bh + 16 + 4 * t); h3 = lds32(bh + 32 + 4 * t);
+            }
+            auto low = [](uint32_t v, uint32_t hb, int i) {
+                return (v & 0x0F0F0F0Fu) | (KIND == FK_Q5_K ? ((hb >> i) & 0x01010101u) << 4 : 0u);
+            };
 #pragma unroll
             for (int j = 0; j < 4; j++) {      // 32 quant bytes: low nibbles = run 2j, high nibbles = run 2j + 1
-                const uint32_t w0 = lds32(bg + 16 + 32 * j + 4 * t), w2 = lds32(bg + 32 + 32 * j + 4 * t);
-                const uint32_t w1 = lds32(bh + 16 + 32 * j + 4 * t), w3 = lds32(bh + 32 + 32 * j + 4 * t);
+                const uint32_t w0 = lds32(bg + QS + 32 * j + 4 * t), w2 = lds32(bg + QS + 16 + 32 * j + 4 * t);
+                const uint32_t w1 = lds32(bh + QS + 32 * j + 4 * t), w3 = lds32(bh + QS + 16 + 32 * j + 4 * t);
                 const int run = u * 8 + 2 * j;
                 const uint32_t xl = xrow + run * 32 + 4 * t;
                 int dl[4], dh4[4];
-                mma_s8(dl, w0 & 0x0F0F0F0Fu, w1 & 0x0F0F0F0Fu, w2 & 0x0F0F0F0Fu, w3 & 0x0F0F0F0Fu, lds32(xl), lds32(xl + 16));
-                mma_s8(dh4, (w0 >> 4) & 0x0F0F0F0Fu, (w1 >> 4) & 0x0F0F0F0Fu, (w2 >> 4) & 0x0F0F0F0Fu, (w3 >> 4) & 0x0F0F0F0Fu, lds32(xl + 32),
-                       lds32(xl + 48));
+                mma_s8(dl, low(w0, h0, 2 * j), low(w1, h1, 2 * j), low(w2, h2, 2 * j), low(w3, h3, 2 * j), lds32(xl), lds32(xl + 16));
+                mma_s8(dh4, low(w0 >> 4, h0, 2 * j + 1), low(w1 >> 4, h1, 2 * j + 1), low(w2 >> 4, h2, 2 * j + 1), low(w3 >> 4, h3, 2 * j + 1),
+                       lds32(xl + 32), lds32(xl + 48));
                 const float2 dxl = *(const float2*)(sdT + run * 8 + 2 * t), dxh = *(const float2*)(sdT + run * 8 + 8 + 2 * t);
                 const float2 sxl = *(const float2*)(ssT + run * 8 + 2 * t), sxh = *(const float2*)(ssT + run * 8 + 8 + 2 * t);
                 const int jb = 2 * (j & 1);
@@ -1198,7 +1211,7 @@ __device__ __forceinline__ void mma_eat(const GemvArgs& a, uint32_t stage, uint3
 // (a block per batch row), not by every block of the matvec: it writes the exact image
 // of the matvec's activation region -- int8 rows `xs` bytes apart (16 more than a row,
 // so the eight batch rows of a B fragment fall on different banks), then the stored
-// scales as [run][8] and, for Q4_K, scale * run sum as [run][8] -- and each matvec
+// scales as [run][8] and, for Q4_K and Q5_K, scale * run sum as [run][8] -- and each matvec
 // block pulls the image in with one bulk copy.  RMSNorm and the gated activation ride
 // here when asked for.
 constexpr int IMG_THREADS = 1024;
@@ -1290,13 +1303,13 @@ __global__ void __launch_bounds__(IMG_THREADS) act_image_kernel(const GemvArgs a
             if (quad == 0) {
                 const float dq = fk_h2f(fk_f2h(d));
                 sdT[kb * 8 + b] = dq;
-                if (KIND == FK_Q4_K) ssT[kb * 8 + b] = dq * (float)qsum;
+                if (MGeo<KIND>::BLOCK) ssT[kb * 8 + b] = dq * (float)qsum;
             }
         }
     }
 }
 
-// The planes of a weight matrix as tensors (Q4_K: one).
+// The planes of a weight matrix as tensors (Q4_K, Q5_K: one).
 struct WeightMaps { CUtensorMap m[4]; };
 
 template <int KIND>
@@ -1355,8 +1368,8 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_mma_kernel(const GemvArg
             const uint32_t p0 = ring + f_stage * a.m_p0_bytes, rest = ring_rest + f_stage * a.m_rest_bytes, bar = bars + 8 * f_stage;
             const int cu0 = u0 + f_ch * a.m_chunk_units, row0 = f_group * MM_ROWS;
             mbar_expect_tx(bar, (uint32_t)a.stage_bytes);
-            if (KIND == FK_Q4_K) {
-                copy2(p0, &wmaps.m[0], cu0 * 36, row0, bar);
+            if (MGeo<KIND>::BLOCK) {
+                copy2(p0, &wmaps.m[0], cu0 * (MGeo<KIND>::BLOCK / 4), row0, bar);
             } else if (KIND == FK_Q6_K) {
                 copy3(p0, &wmaps.m[0], row0, cu0, bar);
                 copy3(rest + a.m_spo[1], &wmaps.m[1], row0, cu0, bar);
@@ -1596,7 +1609,7 @@ int launch_q4k(fk_ctx* ctx, cudaStream_t st, GemvArgs a, const fk_weight_s* w, i
 // stage of one unit does not fit, and the caller falls back to the dp4a form.
 template <int KIND>
 int launch_mma(fk_ctx* ctx, cudaStream_t st, GemvArgs a, const fk_weight_s* w, bool* fits) {
-    constexpr int UNIT = MGeo<KIND>::UNIT;
+    constexpr int UNIT = MGeo<KIND>::UNIT, BLOCK = MGeo<KIND>::BLOCK;
     *fits = false;
     const int units = (a.cols + UNIT - 1) / UNIT, nb32 = a.cols / 32;
     const int ngroups = (a.rows + MM_ROWS - 1) / MM_ROWS;
@@ -1608,7 +1621,7 @@ int launch_mma(fk_ctx* ctx, cudaStream_t st, GemvArgs a, const fk_weight_s* w, b
     size_t act = (size_t)a.batch * a.m_xs;
     act = (act + 15) & ~(size_t)15;
     a.m_sd_off = (int)act;
-    act += (size_t)nb32 * 32 * (KIND == FK_Q4_K ? 2 : 1);
+    act += (size_t)nb32 * 32 * (BLOCK ? 2 : 1);
     act = (act + 15) & ~(size_t)15;
     a.m_red_off = (int)act;
     if (ks > 1) act += 2 * GEMV_WARPS * 32 * 16;
@@ -1621,14 +1634,14 @@ int launch_mma(fk_ctx* ctx, cudaStream_t st, GemvArgs a, const fk_weight_s* w, b
     a.m_d_pitch = (int)w->plane_stride[3];
     // bytes of a stage of cu units: plane 0, then the other planes (512-byte steps keep the swizzled ones aligned)
     auto layout = [&](int cu, GemvArgs& g) {
-        g.m_p0_bytes = KIND == FK_Q4_K ? cu * 144 * MM_ROWS : cu * (KIND == FK_Q6_K ? 1 : 2) * 2048;
+        g.m_p0_bytes = BLOCK ? cu * BLOCK * MM_ROWS : cu * (KIND == FK_Q6_K ? 1 : 2) * 2048;
         int rest = 0;
         g.m_spo[1] = g.m_spo[2] = g.m_spo[3] = 0;
         if (KIND == FK_Q6_K) {
             g.m_spo[2] = rest += cu * 1024;
             g.m_spo[3] = rest += cu * 16 * MM_ROWS;
             rest += MM_ROWS * g.m_d_pitch;
-        } else if (KIND != FK_Q4_K) {
+        } else if (!BLOCK) {
             rest += cu * 16 * MM_ROWS;
         }
         g.stage_bytes = g.m_p0_bytes + rest;
@@ -1636,9 +1649,9 @@ int launch_mma(fk_ctx* ctx, cudaStream_t st, GemvArgs a, const fk_weight_s* w, b
         return g.m_p0_bytes + g.m_rest_bytes;
     };
     int cu = a.m_kpart_units;
-    if (KIND == FK_Q4_K) {
-        if (cu > 7) cu = 7;                 // a tile is at most 256 words wide
-        // rows an odd number of 144-byte blocks apart: the eight rows of a fragment load hit different banks
+    if (BLOCK) {
+        if (cu > (KIND == FK_Q4_K ? 7 : 5)) cu = KIND == FK_Q4_K ? 7 : 5;       // a tile is at most 256 words wide
+        // rows an odd number of 144- or 176-byte blocks apart: the eight rows of a fragment load hit different banks
         if ((cu & 1) == 0) cu--;
         while (cu > 1 && 2 * layout(cu, a) > ring_budget) cu -= 2;
     } else {
@@ -1668,7 +1681,10 @@ int launch_mma(fk_ctx* ctx, cudaStream_t st, GemvArgs a, const fk_weight_s* w, b
     }
     // the activation image lives in the context's scratch block (stream-ordered like its other users)
     const int rcs = fk_ensure_scratch(ctx, st, (size_t)a.m_red_off);
-    if (rcs != FK_OK) return rcs;
+    if (rcs != FK_OK) {
+        *fits = KIND != FK_Q5_K;      // Q5_K's other kernel needs no workspace: it takes a first call under capture
+        return rcs;
+    }
     const uint8_t* img = ctx->scratch;
     const int gpr = GEMV_WARPS / ks;
     int blocks = (ngroups + gpr - 1) / gpr;
@@ -1692,8 +1708,8 @@ int launch_mma(fk_ctx* ctx, cudaStream_t st, GemvArgs a, const fk_weight_s* w, b
     auto plane = [&](int p) { return (void*)(w->dev + (size_t)a.mat * w->mat_stride + w->plane_off[p]); };
     const uint64_t rows = (uint64_t)a.rows;
     int rcm;
-    if (KIND == FK_Q4_K) {
-        rcm = fk_make_map_u32(&maps.m[0], plane(0), w->plane_stride[0] / 4, rows, (uint32_t)(36 * cu), MM_ROWS);
+    if (BLOCK) {
+        rcm = fk_make_map_u32(&maps.m[0], plane(0), w->plane_stride[0] / 4, rows, (uint32_t)(BLOCK / 4 * cu), MM_ROWS);
     } else {
         // plane 0 (and Q6_K's plane 1) as [piece of K][row][piece bytes]: pieces of a row are contiguous, so a ragged last
         // piece reads into the next row (the last row: into the plane's 256 bytes of slack); nothing uses those bytes
@@ -1816,6 +1832,14 @@ int fk_gemv_launch(fk_ctx* ctx, cudaStream_t st, fk_weight w, const int* ids_dev
             // the plain matvec only: the fused, indexed and row-split forms have no Q5_K kernel (the caller composes them
             // from the separate kernels, as it would for any kind this library does not fuse)
             if (ids_dev || n_active_dev || fused) return fk_fail(FK_UNSUPPORTED, "gemv: Q5_K has the plain matvec only");
+            // From two rows on the tensor-core form, whose time does not grow with the batch.  8192x3072: 12.1 us at batch 3 to 8
+            // against 19.9, 31.6 and 55.1 us at batch 2, 4 and 8 of the kernel in fk_gemv_q5k.cu; 1000x4096: 6.2 against
+            // 8.0, 13.4 and 24.2 us; 16384x8192: 33 against 61, 93 and 135 us.  One row: 12.9 us there, nothing to gain.
+            if (batch >= 2 && !dump) {
+                bool fits = false;
+                const int rc = launch_mma<FK_Q5_K>(ctx, st, a, w, &fits);
+                if (fits) return rc;
+            }
             return fk_gemv_q5k_launch(ctx, st, w, mat, x_dev, batch, y_dev, isums_dev);
         case FK_Q6_K: return launch_kind<FK_Q6_K>(ctx, st, a, w, slots, dump);
         case FK_Q8_0: return launch_kind<FK_Q8_0>(ctx, st, a, w, slots, dump);

@@ -1,10 +1,11 @@
 // Q5_K decode matvec (crates/frink-quant/src/lib.rs:424-515, 873-939; block: f16 d, f16 dmin, 12 bytes of
 // 6-bit scales and mins as Q4_K's, 32 bytes qh, 128 bytes of nibbles = 176 bytes per 256 weights).
-// Real Q4_K_M files carry this format in some tensors; it gets the plain matvec (batch 1..8) with the same
+// Real Q4_K_M files carry this format in some tensors; it gets the plain matvec with the same
 // q8_1 activation rule and the same exact per-run integers as the other kinds, not the tuned rings of the
 // Q4_K path: a warp walks the super-blocks of one row four at a time (a lane on 16 nibble bytes = 32 weights),
 // weights read straight from global memory (16-byte loads, every byte once), the quantized activations from
-// shared memory.  HBM-bound on large matrices, latency-bound on small ones.
+// shared memory.  HBM-bound on large matrices, latency-bound on small ones.  One row, the integer hook, and batches that
+// the tensor-core form in fk_gemv.cu cannot take (rows too wide, a workspace that may not grow under capture) run here.
 #include "fk_common.cuh"
 
 namespace {

@@ -1,4 +1,4 @@
-"""The tensor-core matvec (batches of 3 to 8) where its tiled copies are ragged: matrices that end inside a group of 16
+"""The tensor-core matvec (batches of 3 to 8, Q5_K from 2) where its tiled copies are ragged: matrices that end inside a group of 16
 rows, columns that end inside a 128-byte piece, a chunk or a part of K, the second matrix of a stack.  Against the f64
 oracle; the sums are f32 over at most 272 runs, worst case 272 * 2^-24 = 1.6e-5 of the summed magnitudes, for sums of
 random sign well below 1e-5 of the result's norm."""
@@ -10,12 +10,13 @@ from oracle import frink_oracle as fo
 from tests.helpers import rel_l2, synth_acts, synth_weights
 
 pytestmark = pytest.mark.gpu
-COLS = {fo.Q8_0: (32, 288, 2080, 8192), fo.MXFP4: (32, 480, 2880, 8192), fo.Q6_K: (256, 768, 2048, 8192), fo.Q4_K: (256, 768, 2048, 8192)}
+COLS = {fo.Q8_0: (32, 288, 2080, 8192), fo.MXFP4: (32, 480, 2880, 8192), fo.Q6_K: (256, 768, 2048, 8192), fo.Q4_K: (256, 768, 2048, 8192),
+        fo.Q5_K: (256, 768, 2048, 8192)}
 
 
 @pytest.mark.parametrize("kind", list(COLS))
 @pytest.mark.parametrize("ci", range(4))
-@pytest.mark.parametrize("rows,batch", [(1, 3), (15, 8), (17, 5), (1000, 7), (5000, 8)])
+@pytest.mark.parametrize("rows,batch", [(33, 2), (1, 3), (15, 8), (17, 5), (1000, 7), (5000, 8)])
 def test_ragged_tiles(kind, ci, rows, batch):
     from frink_b200 import device
     cols = COLS[kind][ci]
@@ -32,7 +33,7 @@ def test_ragged_tiles(kind, ci, rows, batch):
         assert rel_l2(out[:batch].cpu().numpy(), fo.matmul_f64(kind, raws[m], rows, cols, xq)) <= 1e-5, m
 
 
-@pytest.mark.parametrize("kind,cols,batch", [(fo.Q4_K, 35072, 3), (fo.Q4_K, 19456, 7), (fo.Q8_0, 23232, 5), (fo.Q6_K, 16384, 6),
+@pytest.mark.parametrize("kind,cols,batch", [(fo.Q4_K, 35072, 3), (fo.Q4_K, 19456, 7), (fo.Q5_K, 19200, 7), (fo.Q8_0, 23232, 5), (fo.Q6_K, 16384, 6),
                                              (fo.MXFP4, 23232, 5), (fo.MXFP4, 17440, 7)])
 def test_widest_rows_that_fit(kind, cols, batch):
     """A single stage beside the activations fills shared memory to its last kilobyte."""
