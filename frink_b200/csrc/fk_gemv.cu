@@ -901,7 +901,7 @@ __global__ void __launch_bounds__(Q4_MAX_THREADS, 2) gemv_q4k_kernel(const GemvA
     for (int base = 0; base < items; base += QU * T) {
 #pragma unroll
         for (int u = 0; u < QU; u++) v[u] = nx[u];
-        request(base + QU * T);
+        if (base + QU * T < items) request(base + QU * T);
 #pragma unroll
         for (int u = 0; u < QU; u++) {
             if (base + u * T + warp * 32 >= items) continue;   // nothing for this warp here (the same for all its lanes)
