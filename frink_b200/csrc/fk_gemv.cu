@@ -1832,10 +1832,12 @@ int fk_gemv_launch(fk_ctx* ctx, cudaStream_t st, fk_weight w, const int* ids_dev
             // the plain matvec only: the fused, indexed and row-split forms have no Q5_K kernel (the caller composes them
             // from the separate kernels, as it would for any kind this library does not fuse)
             if (ids_dev || n_active_dev || fused) return fk_fail(FK_UNSUPPORTED, "gemv: Q5_K has the plain matvec only");
-            // From two rows on the tensor-core form, whose time does not grow with the batch.  8192x3072: 12.1 us at batch 3 to 8
-            // against 19.9, 31.6 and 55.1 us at batch 2, 4 and 8 of the kernel in fk_gemv_q5k.cu; 1000x4096: 6.2 against
-            // 8.0, 13.4 and 24.2 us; 16384x8192: 33 against 61, 93 and 135 us.  One row: 12.9 us there, nothing to gain.
-            if (batch >= 2 && !dump) {
+            // From three rows on (as every kind) the tensor-core form, whose time does not grow with the batch.  8192x3072: 12.1 us at
+            // batch 3 to 8 against 31.6 and 55.1 us at batch 4 and 8 of the kernel in fk_gemv_q5k.cu; 1000x4096: 6.2 against 13.4
+            // and 24.2 us; 16384x8192: 33 against 93 and 135 us.  One row: 12.9 us there, nothing to gain.  Two rows (19.9 us
+            // there, 12.1 here) stay there: this form writes its activations to the context's workspace, and a batch of two
+            // is not among the calls that two streams must keep apart.
+            if (batch >= MMA_MIN_BATCH && !dump) {
                 bool fits = false;
                 const int rc = launch_mma<FK_Q5_K>(ctx, st, a, w, &fits);
                 if (fits) return rc;

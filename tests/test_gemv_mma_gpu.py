@@ -1,4 +1,4 @@
-"""The tensor-core matvec (batches of 3 to 8, Q5_K from 2) where its tiled copies are ragged: matrices that end inside a group of 16
+"""The tensor-core matvec (batches of 3 to 8) where its tiled copies are ragged: matrices that end inside a group of 16
 rows, columns that end inside a 128-byte piece, a chunk or a part of K, the second matrix of a stack.  Against the f64
 oracle; the sums are f32 over at most 272 runs, worst case 272 * 2^-24 = 1.6e-5 of the summed magnitudes, for sums of
 random sign well below 1e-5 of the result's norm."""
