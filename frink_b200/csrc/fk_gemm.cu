@@ -556,7 +556,13 @@ __global__ void quantize_acts4_kernel(const float* __restrict__ x, const int* __
     const int t = ok ? (int)(run / nkb) : 0, kb = ok ? (int)(run - (long long)t * nkb) : 0;
     const int src = !ok ? -1 : src_row ? src_row[t] : (t < m ? t : -1);
     float4 f = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (src >= 0) f = __ldg((const float4*)(x + (size_t)src * cols + kb * 32) + part);
+    if (src >= 0) {
+        // every row is whole runs of 128 bytes, so x alone decides whether float4 loads are aligned; the callers may pass a
+        // view that starts at any float
+        const float* p = x + (size_t)src * cols + kb * 32 + part * 4;
+        if (((uintptr_t)x & 15) == 0) f = __ldg((const float4*)p);
+        else f = make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
+    }
     unsigned mb = __float_as_uint(fmaxf(fmaxf(fabsf(f.x), fabsf(f.y)), fmaxf(fabsf(f.z), fabsf(f.w))));
     mb = max(mb, __shfl_xor_sync(0xffffffffu, mb, 1));
     mb = max(mb, __shfl_xor_sync(0xffffffffu, mb, 2));

@@ -1,0 +1,33 @@
+"""What the q8_1 GEMM's entry points take as x: any 4-byte aligned view."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import frink_oracle as fo
+from tests.helpers import synth_acts, synth_weights
+
+pytestmark = pytest.mark.gpu
+KINDS = [fo.Q8_0, fo.Q4_K, fo.Q6_K, fo.MXFP4]
+
+
+def _off(x, n):
+    """A copy of x that starts n floats behind a 16-byte boundary."""
+    v = torch.empty(x.numel() + n, device="cuda")[n:].view(x.shape)
+    assert v.data_ptr() % 16 == 4 * n
+    return v.copy_(x)
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("off", [1, 2, 3])
+def test_x_off_a_16_byte_boundary(kind, off):
+    """The same values at another address: the same bits out."""
+    from frink_b200 import device
+    rows, cols, m, n_exp = 130, 768, 19, 3
+    w = device.Weights(fo.encode(kind, synth_weights(n_exp * rows, cols, 91)), kind, rows, cols, n_mats=n_exp)
+    x = torch.from_numpy(synth_acts(m, cols, 92)).cuda()
+    ids = torch.from_numpy(np.arange(2 * m, dtype=np.int32).reshape(m, 2) % n_exp).cuda()
+    group, gather, _ = device.moe_permute(ids, n_exp)
+    for f in (lambda v: device.gemm(w, v, mat=1), lambda v: device.gemm_static(w, v, mat=1),
+              lambda v: device.gemm_grouped(w, group, gather, v, 2 * m)):
+        assert torch.equal(f(_off(x, off)), f(x))
+    assert device.device_error() == 0
