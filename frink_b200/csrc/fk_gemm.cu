@@ -563,7 +563,9 @@ __global__ void quantize_acts4_kernel(const float* __restrict__ x, const int* __
         if (((uintptr_t)x & 15) == 0) f = __ldg((const float4*)p);
         else f = make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
     }
-    unsigned mb = __float_as_uint(fmaxf(fmaxf(fabsf(f.x), fabsf(f.y)), fmaxf(fabsf(f.z), fabsf(f.w))));
+    // the maximum over bit patterns, as fk_q8_1_lane takes it: a NaN is larger than every number there, so it becomes the run's
+    // scale and reaches the output (fmaxf drops it, and the row came out finite)
+    unsigned mb = max(max(__float_as_uint(fabsf(f.x)), __float_as_uint(fabsf(f.y))), max(__float_as_uint(fabsf(f.z)), __float_as_uint(fabsf(f.w))));
     mb = max(mb, __shfl_xor_sync(0xffffffffu, mb, 1));
     mb = max(mb, __shfl_xor_sync(0xffffffffu, mb, 2));
     mb = max(mb, __shfl_xor_sync(0xffffffffu, mb, 4));

@@ -1,4 +1,5 @@
-"""What the q8_1 GEMM's entry points take as x: any 4-byte aligned view."""
+"""What the q8_1 GEMM's entry points take as x: any 4-byte aligned view, and NaN and infinity, which have to
+reach the output."""
 import numpy as np
 import pytest
 import torch
@@ -30,4 +31,28 @@ def test_x_off_a_16_byte_boundary(kind, off):
     for f in (lambda v: device.gemm(w, v, mat=1), lambda v: device.gemm_static(w, v, mat=1),
               lambda v: device.gemm_grouped(w, group, gather, v, 2 * m)):
         assert torch.equal(f(_off(x, off)), f(x))
+    assert device.device_error() == 0
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), -float("inf")])
+def test_nan_and_infinity_reach_the_output(kind, bad):
+    """A run's scale is the largest magnitude's: NaN or infinite, and so is every output of that token.  Infinity times the
+    codes of the run's finite values, 0, is NaN.  The other tokens keep their bits."""
+    from frink_b200 import device
+    rows, cols, m, n_exp = 130, 768, 19, 3
+    w = device.Weights(fo.encode(kind, synth_weights(n_exp * rows, cols, 93)), kind, rows, cols, n_mats=n_exp)
+    clean = torch.from_numpy(synth_acts(m, cols, 94)).cuda()
+    ids = torch.from_numpy(np.arange(2 * m, dtype=np.int32).reshape(m, 2) % n_exp).cuda()
+    group, gather, _ = device.moe_permute(ids, n_exp)
+    hit = torch.zeros(m, dtype=torch.bool, device="cuda")
+    x = clean.clone()
+    for t, c in ((0, 0), (7, 33), (18, 767), (18, 2)):      # each place in a lane's four values
+        x[t, c] = bad
+        hit[t] = True
+    for f, mask in ((lambda v: device.gemm(w, v, mat=2), hit), (lambda v: device.gemm_static(w, v, mat=2), hit),
+                    (lambda v: device.gemm_grouped(w, group, gather, v, 2 * m), hit[gather.long()])):
+        got, want = f(x), f(clean)
+        assert torch.isnan(got[mask]).all()
+        assert torch.equal(got[~mask], want[~mask])
     assert device.device_error() == 0
