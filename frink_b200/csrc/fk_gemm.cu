@@ -946,11 +946,13 @@ FK_EXPORT int fk_gemm_static(fk_ctx* ctx, void* stream, fk_weight w, int mat, co
     FkDeviceGuard g(ctx->device);
     cudaStream_t st = (cudaStream_t)stream;
     if (w->kind == FK_Q5_K || w->kind == FK_BF16) return fk_fail(FK_UNSUPPORTED, "gemm: kind %d has no kernel", w->kind);
-    // Sized for tiles of 128 tokens whatever tile the plan picks (narrower ones pad less): what fits does not depend on it.
-    const GemmScratch most((m + 127) / 128 * 128, w->cols, 0, false);
-    if (most.total > FK_GEMM_STATIC_BYTES)
+    // Sized for tiles of 128 tokens whatever tile the plan picks (narrower ones pad less), and with two words a padded row as
+    // the row tables of the grouped form take: which shapes fit is part of the interface and does not follow the plan.
+    const int n_most = (m + 127) / 128 * 128;
+    const size_t most = GemmScratch(n_most, w->cols, 0, false).src + 8 * (size_t)n_most;
+    if (most > FK_GEMM_STATIC_BYTES)
         return fk_fail(FK_INVALID, "gemm_static: %d tokens x %d columns needs %zu bytes of scratch, the fixed block holds %zu (use fk_gemm)",
-                       m, w->cols, most.total, (size_t)FK_GEMM_STATIC_BYTES);
+                       m, w->cols, most, (size_t)FK_GEMM_STATIC_BYTES);
     uint8_t* sc = nullptr;
     int rc = static_scratch(ctx, &sc);
     if (rc) return rc;

@@ -1,5 +1,5 @@
 """What the q8_1 GEMM's entry points take as x: any 4-byte aligned view, and NaN and infinity, which have to
-reach the output."""
+reach the output; and what the fixed block of fk_gemm_static holds."""
 import numpy as np
 import pytest
 import torch
@@ -55,4 +55,21 @@ def test_nan_and_infinity_reach_the_output(kind, bad):
         got, want = f(x), f(clean)
         assert torch.isnan(got[mask]).all()
         assert torch.equal(got[~mask], want[~mask])
+    assert device.device_error() == 0
+
+
+@pytest.mark.parametrize("m,cols,fits", [(9600, 512, True), (9601, 512, False), (512, 9824, True), (513, 9824, False), (128, 39296, True), (128, 39328, False)])
+def test_what_the_fixed_block_holds(m, cols, fits):
+    """m padded to 128: m * cols bytes of codes, two scales of 4 bytes a run of 32 (each plane rounded to 1 KB) and two
+    words a row, in 6 MiB."""
+    from frink_b200 import _lib, device
+    w = device.Weights(fo.encode(fo.Q8_0, synth_weights(8, cols, 95)), fo.Q8_0, 8, cols)
+    x, y = torch.from_numpy(synth_acts(m, cols, 96)).cuda(), torch.zeros((m, 8), device="cuda")
+    if fits:
+        assert torch.equal(device.gemm_static(w, x, out=y), device.gemm(w, x))
+    else:
+        with pytest.raises(_lib.Invalid):
+            device.gemm_static(w, x, out=y)
+        torch.cuda.synchronize()
+        assert not y.any()
     assert device.device_error() == 0
