@@ -63,6 +63,7 @@ FK_EXPORT int fk_init(int device, fk_ctx** out) {
     if (e == cudaSuccess) e = cudaMemset(ctx->argmax_cnt, 0, 128 * sizeof(unsigned));
     if (e == cudaSuccess) e = cudaMalloc(&ctx->attn_cnt, 4096 * sizeof(unsigned));
     if (e == cudaSuccess) e = cudaMemset(ctx->attn_cnt, 0, 4096 * sizeof(unsigned));
+    if (e == cudaSuccess) e = cudaMalloc(&ctx->q5k_img, FK_Q5K_IMG_BYTES);
     if (e != cudaSuccess) {
         delete ctx;
         return fk_fail(FK_DRIVER_INIT, "context allocation: %s", cudaGetErrorString(e));
@@ -86,6 +87,7 @@ FK_EXPORT void fk_destroy(fk_ctx* ctx) {
     cudaFree(ctx->argmax_ws);
     cudaFree(ctx->argmax_cnt);
     cudaFree(ctx->attn_cnt);
+    cudaFree(ctx->q5k_img);
     delete ctx;
 }
 

@@ -70,6 +70,9 @@ struct fk_ctx {
     // GEMM / MoE scratch (activation q8_1 planes), grown on demand
     uint8_t* scratch = nullptr;
     size_t scratch_cap = 0;
+    // activation image of the batched Q5_K matvec: its own block, there from fk_init on, so that which kernel a call takes
+    // depends on its shape alone and not on whether the scratch block has been allocated yet (it cannot be under capture)
+    uint8_t* q5k_img = nullptr;
     std::vector<uint8_t*> scratch_retired;   // outgrown blocks: queued launches and captured graphs may still name them
     // device word kernels raise when a bounded wait gives up
     int* err_flag = nullptr;       // 16 bytes on the device: the error word, and at byte 8 the device address of its host mirror
@@ -142,6 +145,7 @@ int fk_gemv_multi_gate_up_launch(fk_ctx* ctx, void* stream, fk_weight gate, fk_w
 int fk_gemv_launch(fk_ctx* ctx, cudaStream_t st, fk_weight w, const int* ids_dev, int mat, int slots,
                    const float* x_dev, int x_stride, int batch, float* y_dev, int32_t* isums_dev, const int* n_active_dev,
                    const FkGemvFused* fused);
+constexpr size_t FK_Q5K_IMG_BYTES = (size_t)256 << 10;   // an image fits one SM's shared memory
 constexpr size_t FK_SCRATCH_MIN = (size_t)64 << 20;
 int fk_ensure_scratch(fk_ctx* ctx, cudaStream_t st, size_t bytes);
 int fk_gemv_bf16_launch(fk_ctx* ctx, cudaStream_t st, fk_weight w, int mat, const float* x_dev, int x_ld, int batch, float* y_dev,

@@ -1679,13 +1679,14 @@ int launch_mma(fk_ctx* ctx, cudaStream_t st, GemvArgs a, const fk_weight_s* w, b
             granted[dev].store((int)smem, std::memory_order_relaxed);
         }
     }
-    // the activation image lives in the context's scratch block (stream-ordered like its other users)
-    const int rcs = fk_ensure_scratch(ctx, st, (size_t)a.m_red_off);
-    if (rcs != FK_OK) {
-        *fits = KIND != FK_Q5_K;      // Q5_K's other kernel needs no workspace: it takes a first call under capture
-        return rcs;
+    // the activation image: in the context's scratch block (stream-ordered like its other users), Q5_K's in a block of its own
+    static_assert(SMEM_BUDGET + MMA_ALIGN <= FK_Q5K_IMG_BYTES, "an image is smaller than the shared memory it is copied to");
+    uint8_t* img = ctx->q5k_img;
+    if (KIND != FK_Q5_K) {
+        const int rcs = fk_ensure_scratch(ctx, st, (size_t)a.m_red_off);
+        if (rcs != FK_OK) return rcs;
+        img = ctx->scratch;
     }
-    const uint8_t* img = ctx->scratch;
     const int gpr = GEMV_WARPS / ks;
     int blocks = (ngroups + gpr - 1) / gpr;
     if (blocks > ctx->sm_count) blocks = ctx->sm_count;
@@ -1724,8 +1725,8 @@ int launch_mma(fk_ctx* ctx, cudaStream_t st, GemvArgs a, const fk_weight_s* w, b
         }
     }
     if (rcm != FK_OK) return rcm;
-    FK_CUDA(cudaLaunchKernelEx(&icfg, act_image_kernel<KIND>, a, ctx->scratch), FK_LAUNCH);
-    FK_CUDA(cudaLaunchKernelEx(&cfg, kern, a, img, maps), FK_LAUNCH);
+    FK_CUDA(cudaLaunchKernelEx(&icfg, act_image_kernel<KIND>, a, img), FK_LAUNCH);
+    FK_CUDA(cudaLaunchKernelEx(&cfg, kern, a, (const uint8_t*)img, maps), FK_LAUNCH);
     ctx->launches += 2;
     return FK_OK;
 }
@@ -1835,7 +1836,7 @@ int fk_gemv_launch(fk_ctx* ctx, cudaStream_t st, fk_weight w, const int* ids_dev
             // From three rows on (as every kind) the tensor-core form, whose time does not grow with the batch.  8192x3072: 12.1 us at
             // batch 3 to 8 against 31.6 and 55.1 us at batch 4 and 8 of the kernel in fk_gemv_q5k.cu; 1000x4096: 6.2 against 13.4
             // and 24.2 us; 16384x8192: 33 against 93 and 135 us.  One row: 12.9 us there, nothing to gain.  Two rows (19.9 us
-            // there, 12.1 here) stay there: this form writes its activations to the context's workspace, and a batch of two
+            // there, 12.1 here) stay there: this form keeps its activations in one block of the context, and a batch of two
             // is not among the calls that two streams must keep apart.
             if (batch >= MMA_MIN_BATCH && !dump) {
                 bool fits = false;

@@ -4,8 +4,8 @@
 // q8_1 activation rule and the same exact per-run integers as the other kinds, not the tuned rings of the
 // Q4_K path: a warp walks the super-blocks of one row four at a time (a lane on 16 nibble bytes = 32 weights),
 // weights read straight from global memory (16-byte loads, every byte once), the quantized activations from
-// shared memory.  HBM-bound on large matrices, latency-bound on small ones.  One row, the integer hook, and batches that
-// the tensor-core form in fk_gemv.cu cannot take (rows too wide, a workspace that may not grow under capture) run here.
+// shared memory.  HBM-bound on large matrices, latency-bound on small ones.  One row, two rows, the integer hook, and
+// batches whose rows are too wide for the tensor-core form in fk_gemv.cu run here.
 #include "fk_common.cuh"
 
 namespace {
