@@ -20,9 +20,10 @@
 //               weight tile itself for Q8_0, whose int8 plane needs no unpacking)
 //   MMA issuer  one elected lane, + TMEM allocation
 // The CTAs of a cluster may share one tile, each on its own part of K; their f32 sums meet in distributed shared memory.
-// Stages (K = 128 each) and TMEM accumulators are rings guarded by mbarriers;
-// every wait is bounded and raises the context's error word instead of
-// spinning forever.
+// Stages (K = 128 each) and TMEM accumulators are rings guarded by mbarriers; every mbarrier wait is bounded and raises
+// the context's error word instead of spinning forever.  Two waits have no limit of their own: the cluster barriers of a
+// split tile, which every CTA reaches because its mbarrier waits end, and tcgen05.alloc, which never has to wait for a
+// CTA that waits for others (see the co-residence asserts below Smem).
 #include "fk_common.cuh"
 
 #include <math.h>
@@ -85,9 +86,21 @@ template <int BN> struct Smem {
     static constexpr int DX = A_BYTES + B_BYTES, DW = DX + 2 * DX_BYTES;
     static constexpr int STAGE = DW + 2 * DW_BYTES;
     static constexpr int BARS = NSTAGE * STAGE;          // barrier block
-    static constexpr int TOTAL = BARS + 256 + 1024;      // + alignment slack
+    static constexpr int USED = BARS + 256 + 1024;       // + alignment slack
+    static constexpr int TOTAL = BN == 64 && USED < 128 * 1024 ? 128 * 1024 : USED;   // 64: see below
     static_assert(BM * BN * 4 <= BARS, "the partial sums of a split tile reuse the stages");
 };
+
+// A CTA of a split tile waits for its cluster while it holds tensor memory.  Were CTAs of two such grids (two contexts, two
+// streams) to meet on two SMs whose tensor memory holds one of them, each could hold what the other's cluster waits for, for
+// ever.  So CTAs that share an SM must fit its tensor memory together: what does not fit is kept off by its shared memory
+// (the 64-token tile asks for 4 KB more than it uses).  Two 32-token tiles fit both; three fit neither.
+constexpr int SM_SMEM = 228 * 1024, CTA_RESERVED = 1024, TMEM_COLS = 512;
+template <int A, int B> constexpr bool may_share_an_sm() { return Smem<A>::TOTAL + Smem<B>::TOTAL + 2 * CTA_RESERVED <= SM_SMEM; }
+template <int BN> constexpr int tmem_cols() { return Tile<BN>::NACC * BN; }
+static_assert(!may_share_an_sm<128, 128>() && !may_share_an_sm<128, 64>() && !may_share_an_sm<128, 32>() && !may_share_an_sm<64, 64>() &&
+              !may_share_an_sm<64, 32>(), "their accumulators do not fit one SM's tensor memory");
+static_assert(may_share_an_sm<32, 32>() && 2 * tmem_cols<32>() <= TMEM_COLS && 3 * (Smem<32>::TOTAL + CTA_RESERVED) > SM_SMEM, "two 32-token tiles, not three");
 
 // The weight scales of one tile row for one stage (runs kb0 .. kb0 + 3): as loaded, and decoded.  The unpack warps load
 // them beside the row they belong to and leave them decoded in the stage, so the epilogue -- the kernel's critical path --
