@@ -98,9 +98,14 @@ struct GemvArgs {
     int m_xs;              // bytes between batch rows of the quantized activations
     int m_sd_off, m_red_off;
     int m_p0_bytes, m_rest_bytes;   // a stage's plane 0, its other planes
-    int m_spo[4];             // offset of planes 1.. inside the rest
-    int m_d_pitch;            // Q6_K: bytes between rows of the super-scales
+    int m_spo[3];             // offsets of planes 1, 2 and 3 inside the rest
 };
+
+// A kernel parameter block above 424 bytes costs a call 0.5 us more (432, 440 and 496 bytes measured alike): the host-buffer
+// matvec of 3072x3072 Q4_K 25.3 us a call at 424 bytes, 25.9 at 432.
+#ifndef FK_TRACE
+static_assert(sizeof(GemvArgs) <= 424, "the step in the cost of a launch");
+#endif
 
 // ------------------------------------------------------------------ PTX glue
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -883,7 +888,8 @@ __global__ void __launch_bounds__(Q4_MAX_THREADS, 2) gemv_q4k_kernel(const GemvA
     const int c4 = cols >> 2, items = NB * c4;
     constexpr int QU = 1024 / Q4_MAX_THREADS;
     // the next pass over x is requested before this one is quantized: with 8192 columns (two passes) the second wait for L2
-    // came on top of the first (with the odd pitch of the partial sums, 3072x8192: 7.1 -> 6.1 us a launch)
+    // came on top of the first.  Rows of one pass gain by this form of the loop, too.  A launch in a chain of them: 8192x3072
+    // 4.81 -> 4.08 us, 3072x3072 4.20 -> 3.94, 3072x8192 7.09 -> 6.92; with the odd pitch of the partial sums 4.02, 3.89, 6.17
     float4 v[QU], nx[QU];
     auto request = [&](int base) {
 #pragma unroll
@@ -1126,7 +1132,7 @@ __device__ __forceinline__ void mma_eat(const GemvArgs& a, uint32_t stage, uint3
             }
         }
     } else if (KIND == FK_Q8_0) {
-        const uint32_t s0 = rest + a.m_spo[1] + g * spitch, s8 = s0 + 8 * spitch;
+        const uint32_t s0 = rest + a.m_spo[0] + g * spitch, s8 = s0 + 8 * spitch;
         for (int u = cu0; u < cu1; u++) {
 #pragma unroll
             for (int r = 0; r < 8; r++) {
@@ -1146,7 +1152,7 @@ __device__ __forceinline__ void mma_eat(const GemvArgs& a, uint32_t stage, uint3
             }
         }
     } else if (KIND == FK_MXFP4) {
-        const uint32_t s0 = rest + a.m_spo[1] + g * spitch, s8 = s0 + 8 * spitch;
+        const uint32_t s0 = rest + a.m_spo[0] + g * spitch, s8 = s0 + 8 * spitch;
         for (int u = cu0; u < cu1; u++) {
 #pragma unroll 4
             for (int r = 0; r < 16; r++) {
@@ -1167,9 +1173,9 @@ __device__ __forceinline__ void mma_eat(const GemvArgs& a, uint32_t stage, uint3
             }
         }
     } else {   // FK_Q6_K
-        const uint32_t h0 = rest + a.m_spo[1] + g * 64 + 4 * t;            // row g + 8 is 512 bytes further on
-        const uint32_t c0 = rest + a.m_spo[2] + g * spitch, c8 = c0 + 8 * spitch;
-        const uint32_t d0 = rest + a.m_spo[3] + g * a.m_d_pitch, d8 = d0 + 8 * a.m_d_pitch;
+        const uint32_t h0 = rest + a.m_spo[0] + g * 64 + 4 * t;            // row g + 8 is 512 bytes further on
+        const uint32_t c0 = rest + a.m_spo[1] + g * spitch, c8 = c0 + 8 * spitch;
+        const uint32_t d_pitch = (uint32_t)a.plane_stride[3], d0 = rest + a.m_spo[2] + g * d_pitch, d8 = d0 + 8 * d_pitch;
         for (int u = cu0; u < cu1; u++) {
             const float dg = fk_h2f((uint16_t)lds_u16(d0 + u * 2)), dh = fk_h2f((uint16_t)lds_u16(d8 + u * 2));   // the whole row's super-scales are staged
             const uint4 scg = lds16(c0 + (u - cu0) * 16), sch = lds16(c8 + (u - cu0) * 16);
@@ -1372,12 +1378,12 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_mma_kernel(const GemvArg
                 copy2(p0, &wmaps.m[0], cu0 * (MGeo<KIND>::BLOCK / 4), row0, bar);
             } else if (KIND == FK_Q6_K) {
                 copy3(p0, &wmaps.m[0], row0, cu0, bar);
-                copy3(rest + a.m_spo[1], &wmaps.m[1], row0, cu0, bar);
-                copy2(rest + a.m_spo[2], &wmaps.m[2], cu0 * 16, row0, bar);
-                copy2(rest + a.m_spo[3], &wmaps.m[3], 0, row0, bar);          // the whole row's super-scales
+                copy3(rest + a.m_spo[0], &wmaps.m[1], row0, cu0, bar);
+                copy2(rest + a.m_spo[1], &wmaps.m[2], cu0 * 16, row0, bar);
+                copy2(rest + a.m_spo[2], &wmaps.m[3], 0, row0, bar);          // the whole row's super-scales
             } else {
                 copy3(p0, &wmaps.m[0], row0, 2 * cu0, bar);
-                copy2(rest + a.m_spo[1], &wmaps.m[1], cu0 * 16, row0, bar);
+                copy2(rest + a.m_spo[0], &wmaps.m[1], cu0 * 16, row0, bar);
             }
         }
         if (++f_stage == a.nstages) f_stage = 0;
@@ -1631,16 +1637,15 @@ int launch_mma(fk_ctx* ctx, cudaStream_t st, GemvArgs a, const fk_weight_s* w, b
     // 227 KB in all: the widest rows still fit
     const int ring_budget = ((int)SMEM_BUDGET + MMA_ALIGN - (int)act - bars) / GEMV_WARPS;
     if (KIND == FK_Q6_K && w->plane_stride[3] > 256) return FK_UNSUPPORTED;      // a row's super-scales are one box row of at most 256 bytes
-    a.m_d_pitch = (int)w->plane_stride[3];
     // bytes of a stage of cu units: plane 0, then the other planes (512-byte steps keep the swizzled ones aligned)
     auto layout = [&](int cu, GemvArgs& g) {
         g.m_p0_bytes = BLOCK ? cu * BLOCK * MM_ROWS : cu * (KIND == FK_Q6_K ? 1 : 2) * 2048;
         int rest = 0;
-        g.m_spo[1] = g.m_spo[2] = g.m_spo[3] = 0;
+        g.m_spo[0] = g.m_spo[1] = g.m_spo[2] = 0;
         if (KIND == FK_Q6_K) {
-            g.m_spo[2] = rest += cu * 1024;
-            g.m_spo[3] = rest += cu * 16 * MM_ROWS;
-            rest += MM_ROWS * g.m_d_pitch;
+            g.m_spo[1] = rest += cu * 1024;
+            g.m_spo[2] = rest += cu * 16 * MM_ROWS;
+            rest += MM_ROWS * (int)w->plane_stride[3];
         } else if (!BLOCK) {
             rest += cu * 16 * MM_ROWS;
         }
