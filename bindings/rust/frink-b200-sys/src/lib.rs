@@ -235,6 +235,28 @@ extern "C" {
         out_dev: *mut f32,
         isums_dev: *mut i32,
     ) -> c_int;
+    pub fn fk_gemm_plan(
+        ctx: *mut FkCtx,
+        w: FkWeight,
+        m: c_int,
+        grouped: c_int,
+        tile: *mut c_int,
+        split: *mut c_int,
+    ) -> c_int;
+    pub fn fk_gemm_tiled(
+        ctx: *mut FkCtx,
+        stream: *mut c_void,
+        w: FkWeight,
+        mat: c_int,
+        group_off_dev: *const c_int,
+        gather_dev: *const c_int,
+        x_dev: *const f32,
+        m: c_int,
+        out_dev: *mut f32,
+        isums_dev: *mut i32,
+        tile: c_int,
+        split: c_int,
+    ) -> c_int;
     pub fn fk_gemm_q8k(
         ctx: *mut FkCtx,
         stream: *mut c_void,

@@ -47,6 +47,8 @@ SYMBOLS = {
     "fk_gemv_isums": (_I, [_P, _P, _P, _I, _P, _P]),
     "fk_gemm": (_I, [_P, _P, _P, _I, _P, _I, _P]),
     "fk_gemm_isums": (_I, [_P, _P, _P, _I, _P, _I, _P, _P]),
+    "fk_gemm_plan": (_I, [_P, _P, _I, _I, C.POINTER(_I), C.POINTER(_I)]),
+    "fk_gemm_tiled": (_I, [_P, _P, _P, _I, _P, _P, _P, _I, _P, _P, _I, _I]),
     "fk_gemm_q8k": (_I, [_P, _P, _P, _I, _P, _I, _P]),
     "fk_gemm_q8k_isums": (_I, [_P, _P, _P, _I, _P, _I, _P, _P]),
     "fk_gemm_static": (_I, [_P, _P, _P, _I, _P, _I, _P]),

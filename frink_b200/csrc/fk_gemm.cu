@@ -745,8 +745,8 @@ int launch_by_kind(fk_ctx* ctx, cudaStream_t st, const GemmArgs& a, int kind, co
 //
 //   waves * (runs / split * us_per_run(bn) + (split > 1) * exchange(bn)),   waves = CTAs / (SMs * CTAs per SM)
 //
-// The constants were measured on B200 (us; Q4_K, 3072 x 3072, cold L2; the other kinds are within 20 % below): a 128-token
-// tile takes 0.68 a run of 32 K, a 64-token one 0.47, a 32-token one 0.42 alone on its SM and 0.56 beside another; the parts
+// The constants were measured on B200 (us; Q4_K, 3072 x 3072, cold L2; the other kinds are within 20 % below, but MXFP4 in
+// 128-token tiles takes 0.80): a 128-token tile takes 0.68 a run of 32 K, a 64-token one 0.47, a 32-token one 0.42 alone on its SM and 0.56 beside another; the parts
 // of a split tile take 6 to 8 to meet.  A tile's own time falls far less than its width -- its warps walk the same chain per
 // run -- so what a short prompt needs is more CTAs, not only narrower ones: 3072 x 3072, M = 128 was 24 CTAs and 95 us, and
 // is 96 CTAs and 32 us; 3072 x 8192 Q6_K, M = 77 204 -> 77 us; 512 x 3072, M = 16 93 -> 17 us; 8192 x 3072, M = 512 keeps
@@ -834,13 +834,13 @@ int gemm_run(fk_ctx* ctx, cudaStream_t st, fk_weight w, int mat, const float* x,
                       : launch_by_kind<32>(ctx, st, a, w->kind, mq, mdx, msx, mw, tiles);
 }
 
-// Shared body of fk_gemm (group_off == nullptr) and fk_gemm_grouped.
+// Shared body of fk_gemm (group_off == nullptr) and fk_gemm_grouped; `given` takes the place of the plan (test hook).
 int gemm_common(fk_ctx* ctx, cudaStream_t st, fk_weight w, int mat, const int* group_off, const int* gather, const float* x,
-                int n_tokens, float* out, int32_t* isums = nullptr) {
+                int n_tokens, float* out, int32_t* isums = nullptr, const GemmPlan* given = nullptr) {
     const bool grouped = group_off != nullptr;
     if (w->kind == FK_Q5_K || w->kind == FK_BF16)   // before anything is enqueued: the caller takes batches of 8 through the matvec
         return fk_fail(FK_UNSUPPORTED, "gemm: kind %d has the plain matvec only", w->kind);
-    const GemmPlan plan = gemm_plan(ctx, w, n_tokens, grouped);
+    const GemmPlan plan = given ? *given : gemm_plan(ctx, w, n_tokens, grouped);
     const int n_tiles_max = (n_tokens + plan.bn - 1) / plan.bn + (grouped ? w->n_mats : 0), n_pad = n_tiles_max * plan.bn;
     const GemmScratch L(n_pad, w->cols, n_tiles_max, grouped);
     int rc = fk_ensure_scratch(ctx, st, L.total);
@@ -909,6 +909,29 @@ FK_EXPORT int fk_gemm_isums(fk_ctx* ctx, void* stream, fk_weight w, int mat, con
     if (mat < 0 || mat >= w->n_mats) return fk_fail(FK_INVALID, "gemm_isums: matrix %d of %d", mat, w->n_mats);
     FkDeviceGuard g(ctx->device);
     return gemm_common(ctx, (cudaStream_t)stream, w, mat, nullptr, nullptr, x_dev, m, out_dev, isums_dev);
+}
+
+FK_EXPORT int fk_gemm_plan(fk_ctx* ctx, fk_weight w, int m, int grouped, int* tile, int* split) {
+    if (!ctx || !w || !tile || !split) return fk_fail(FK_INVALID, "gemm_plan: null argument");
+    if (m < 1) return fk_fail(FK_INVALID, "gemm_plan: m=%d", m);
+    const GemmPlan plan = gemm_plan(ctx, w, m, grouped != 0);
+    *tile = plan.bn;
+    *split = plan.split;
+    return FK_OK;
+}
+
+FK_EXPORT int fk_gemm_tiled(fk_ctx* ctx, void* stream, fk_weight w, int mat, const int* group_off_dev, const int* gather_dev, const float* x_dev, int m,
+                            float* out_dev, int32_t* isums_dev, int tile, int split) {
+    if (!ctx || !w || !x_dev || !out_dev) return fk_fail(FK_INVALID, "gemm_tiled: null argument");
+    if (m < 1) return fk_fail(FK_INVALID, "gemm_tiled: m=%d", m);
+    if (mat < 0 || mat >= w->n_mats) return fk_fail(FK_INVALID, "gemm_tiled: matrix %d of %d", mat, w->n_mats);
+    if (tile != 128 && tile != 64 && tile != 32) return fk_fail(FK_INVALID, "gemm_tiled: tile %d", tile);
+    const int stages = (w->cols + KSTAGE - 1) / KSTAGE;
+    if (split < 1 || split > MAX_SPLIT || (split & (split - 1)) || split > stages)
+        return fk_fail(FK_INVALID, "gemm_tiled: %d parts of %d stages", split, stages);
+    FkDeviceGuard g(ctx->device);
+    const GemmPlan plan{tile, split};
+    return gemm_common(ctx, (cudaStream_t)stream, w, mat, group_off_dev, gather_dev, x_dev, m, out_dev, isums_dev, &plan);
 }
 
 FK_EXPORT int fk_gemm_grouped(fk_ctx* ctx, void* stream, fk_weight w, const int* group_off_dev, const int* gather_dev,

@@ -327,6 +327,23 @@ def gemm_isums(w, x, mat=0):
     return y, isums
 
 
+def gemm_plan(w, m, grouped=False):
+    """(tile, split) that `gemm` or `gemm_grouped` picks for m rows: tokens a CTA covers, CTAs along the columns."""
+    tile, split = C.c_int(), C.c_int()
+    check(lib().fk_gemm_plan(w._ctx, w.handle, m, int(grouped), C.byref(tile), C.byref(split)))
+    return tile.value, split.value
+
+
+def gemm_tiled(w, x, tile, split, mat=0, group_off=None, gather=None, pairs=None, isums=False):
+    """`gemm` (or, with group_off, `gemm_grouped` over `pairs` rows) with a given plan; isums: (out, the integers of `gemm_isums`)."""
+    x = _f32(x)
+    m = x.shape[0] if group_off is None else pairs
+    y = torch.empty((m, w.rows), dtype=torch.float32, device=x.device)
+    s = torch.empty((m, w.rows, w.cols // (16 if w.kind == 14 else 32)), dtype=torch.int32, device=x.device) if isums else None
+    check(lib().fk_gemm_tiled(w._ctx, _stream(), w.handle, mat, _ptr(group_off), _ptr(gather), _ptr(x), m, _ptr(y), _ptr(s), tile, split))
+    return (y, s) if isums else y
+
+
 def gemm_q8k(w, x, mat=0, out=None):
     """out[t, r] = W[mat][r] . q8_k(x[t]): the GEMM on frink's CPU activation rule (Q4_K weights)."""
     x = _f32(x)

@@ -173,7 +173,10 @@ int fk_gemv_isums(fk_ctx* ctx, void* stream, fk_weight w, int mat, const float* 
 /* ---- prefill GEMM ---------------------------------------------------------
  * Replaces `mul_mm_launch::launch_mul_mm` / `enqueue_mmq` (crates/frink-cuda/
  * src/mul_mm_launch.rs:40-68, src/mmq/mod.rs:30-133):
- * out_dev[t * rows + r] = W[mat][r] . q8_1(x_dev[t * cols ..]),  0 <= t < m. */
+ * out_dev[t * rows + r] = W[mat][r] . q8_1(x_dev[t * cols ..]),  0 <= t < m.
+ * A call repeats bit for bit.  The columns may be summed in 2, 4 or 8 parts whose sums are then added in order; how many
+ * depends on the shape, m included, so a token's last bits may differ between a prompt fed whole and one fed in pieces (they
+ * do not depend on what else is in the call at the same m).  x_dev: any float address. */
 int fk_gemm(fk_ctx* ctx, void* stream, fk_weight w, int mat, const float* x_dev, int m, float* out_dev);
 
 /* Test hook, the GEMM's counterpart of fk_gemv_isums (the reference's GEMM twins expose the
@@ -181,6 +184,14 @@ int fk_gemm(fk_ctx* ctx, void* stream, fk_weight w, int mat, const float* x_dev,
  * exact int32 dot of every run of 32 activations (16 for Q6_K) as the tensor cores
  * delivered it, before any scale: isums_dev is [m][rows][cols / run]. */
 int fk_gemm_isums(fk_ctx* ctx, void* stream, fk_weight w, int mat, const float* x_dev, int m, float* out_dev, int32_t* isums_dev);
+
+/* Test hooks: the tile plan that fk_gemm (grouped 0) or fk_gemm_grouped (1) picks for m rows -- tokens a CTA covers (128, 64
+ * or 32) and CTAs that share a tile, each on its part of the columns (1, 2, 4 or 8) -- and the same GEMM with a given plan:
+ * dense when group_off_dev is null, else grouped over m pairs (gather_dev as there); isums_dev (optional) as in
+ * fk_gemm_isums. */
+int fk_gemm_plan(fk_ctx* ctx, fk_weight w, int m, int grouped, int* tile, int* split);
+int fk_gemm_tiled(fk_ctx* ctx, void* stream, fk_weight w, int mat, const int* group_off_dev, const int* gather_dev, const float* x_dev, int m,
+                  float* out_dev, int32_t* isums_dev, int tile, int split);
 
 /* The prefill GEMM on frink's CPU activation rule: Q8_K activations (one f32 scale and sixteen
  * 16-value sums per 256 values, `quantize_activations_q8_k`, crates/frink-quant/src/act_quant.rs:

@@ -24,3 +24,19 @@ def test_block_heights(n_q, n_heads, n_kv, hd, p0, window):
     out = device.attention(q.cuda(), kc.cuda(), vc.cuda(), n_heads, n_kv, hd, pos.cuda(), window=window)
     assert rel_l2(out.cpu().numpy(), want) <= 2e-6
     assert device.device_error() == 0
+
+
+@pytest.mark.parametrize("n_q,n_heads,n_kv", [(16, 8, 8), (75, 64, 8), (150, 32, 8), (333, 64, 8)])
+def test_block_heights_with_sinks(n_q, n_heads, n_kv):
+    """gpt-oss's logit per head in the denominator, under its window and without one."""
+    from frink_b200 import device
+    from tests import cpu_ops
+    rng, hd, p0 = np.random.default_rng(42 + n_q), 64, 5
+    rnd = lambda *s: torch.from_numpy(rng.standard_normal(s).astype(np.float32))
+    q, kc, vc, sinks = rnd(n_q, n_heads * hd), rnd(p0 + n_q, n_kv * hd), rnd(p0 + n_q, n_kv * hd), rnd(n_heads)
+    pos = torch.tensor([p0], dtype=torch.int32)
+    for window in (0, 128):
+        want = cpu_ops.attention(q, kc, vc, n_heads, n_kv, hd, pos, window=window, sinks=sinks).numpy()
+        out = device.attention(q.cuda(), kc.cuda(), vc.cuda(), n_heads, n_kv, hd, pos.cuda(), window=window, sinks=sinks.cuda())
+        assert rel_l2(out.cpu().numpy(), want) <= 2e-6
+    assert device.device_error() == 0

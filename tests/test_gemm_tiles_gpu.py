@@ -15,11 +15,11 @@ KINDS = [fo.Q8_0, fo.Q4_K, fo.Q6_K, fo.MXFP4]
 
 @pytest.mark.parametrize("kind", KINDS)
 @pytest.mark.parametrize("rows,cols,m", [
-    (1, 512, 9),            # one weight row, two to four stages over the parts
+    (1, 512, 9),            # one weight row, one CTA
     (130, 1280, 31), (130, 1280, 33),     # ten stages over eight parts; a 32-token tile short of one, over by one
     (640, 8192, 16),        # the deepest split
-    (2100, 768, 65), (3100, 512, 129),    # wide matrices: no split, ragged 64- and 128-token tiles
-    (1030, 2048, 300)])
+    (2100, 768, 65), (3100, 512, 129),    # wide matrices: no split, ragged 32-token tiles (Q6_K, 129 tokens: 64)
+    (1030, 2048, 300)])     # 128-token tiles in two (Q6_K) or four parts
 def test_tiles_and_parts_of_k(kind, rows, cols, m):
     from frink_b200 import device
     raw = fo.encode(kind, synth_weights(rows, cols, 31 + rows))
@@ -69,3 +69,95 @@ def test_grouped_tiles(kind, n_exp, rows, cols, batch, k):
         lo, hi = off_h[e], off_h[e + 1]
         if hi > lo:
             assert rel_l2(got[lo:hi], fo.matmul_f64(kind, raws[e], rows, cols, xq[gather_h[lo:hi]])) <= 1e-5, e
+
+
+# ---- every tile and split, whatever the plan would pick ----
+def _cols(kind, split):
+    """Nine stages and more in every part (the ring of four wraps twice, the slots of the unpack warps rotate through), parts
+    of unequal length, and the last stage ragged where the kind allows it."""
+    return 1280 * split + (0 if kind in (fo.Q4_K, fo.Q6_K) else 32)
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("tile", [32, 64, 128])
+@pytest.mark.parametrize("split", [1, 2, 4, 8])
+def test_given_plan(kind, tile, split):
+    """Results and raw integers of a given plan on ragged rows and tokens.  At most 322 runs summed in f32 (x 2 halves for Q6_K):
+    worst case 3.8e-5 of the summed magnitudes, for sums of random sign well below 1e-5 of the result's norm."""
+    from frink_b200 import device
+    rows, cols, m = 150, _cols(kind, split), tile + 13
+    raw, x = fo.encode(kind, synth_weights(rows, cols, 101)), synth_acts(m, cols, 102)
+    w, xd = device.Weights(raw, kind, rows, cols), torch.from_numpy(x).cuda()
+    got = device.gemm_tiled(w, xd, tile, split)
+    assert rel_l2(got.cpu().numpy(), fo.matmul_f64(kind, raw, rows, cols, fo.q8_1_round(x))) <= 1e-5
+    with_ints, isums = device.gemm_tiled(w, xd, tile, split, isums=True)
+    assert torch.equal(with_ints, got) and device.device_error() == 0
+    for t in (0, 1, tile - 1, tile, m - 1):
+        assert np.array_equal(isums[t].cpu().numpy(), fo.matrix_isums(kind, raw, rows, cols, fo.quantize_q8_1(x[t]))), f"token {t}"
+    # the order of the sums follows the split alone: not the tile, nor how many tokens are in the call
+    assert torch.equal(device.gemm_tiled(w, xd[:9], 32, split), got[:9])
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("tile,split", [(32, 1), (64, 1), (128, 1), (32, 4), (64, 2), (128, 2)])
+def test_given_plan_grouped(kind, tile, split):
+    """Experts with no row, one row, one over a tile; columns as above."""
+    from frink_b200 import device
+    rows, cols, sizes = 150, _cols(kind, split), [0, 1, tile + 1, 0, 7, tile]
+    pairs = sum(sizes)
+    raws = [fo.encode(kind, synth_weights(rows, cols, 110 + e)) for e in range(len(sizes))]
+    w = device.Weights(np.concatenate(raws), kind, rows, cols, n_mats=len(sizes))
+    x = synth_acts(40, cols, 103)
+    off = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int32)
+    gather = np.random.default_rng(104).integers(0, 40, pairs).astype(np.int32)
+    xd, offd, gd = torch.from_numpy(x).cuda(), torch.from_numpy(off).cuda(), torch.from_numpy(gather).cuda()
+    got = device.gemm_tiled(w, xd, tile, split, group_off=offd, gather=gd, pairs=pairs).cpu().numpy()
+    assert device.device_error() == 0
+    xq = fo.q8_1_round(x)
+    for e in range(len(sizes)):
+        lo, hi = off[e], off[e + 1]
+        if hi > lo:
+            assert rel_l2(got[lo:hi], fo.matmul_f64(kind, raws[e], rows, cols, xq[gather[lo:hi]])) <= 1e-5, e
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("rows,cols,m", [(8192, 512, 512), (1030, 2048, 300), (640, 2048, 16), (2100, 768, 65)])
+def test_the_call_runs_its_plan(kind, rows, cols, m):
+    from frink_b200 import _lib, device
+    w = device.Weights(fo.encode(kind, synth_weights(rows, cols, 105)), kind, rows, cols)
+    x = torch.from_numpy(synth_acts(m, cols, 106)).cuda()
+    tile, split = device.gemm_plan(w, m)
+    assert tile in (32, 64, 128) and split in (1, 2, 4, 8) and split * 128 <= cols
+    want = device.gemm_tiled(w, x, tile, split)
+    assert torch.equal(device.gemm(w, x), want) and torch.equal(device.gemm_static(w, x), want)
+    for bad in ((48, 1), (32, 3), (32, 16), (32, 0)):
+        with pytest.raises(_lib.Invalid):
+            device.gemm_tiled(w, x, *bad)
+    assert device.device_error() == 0
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("rows,cols,m", [(300, 1280, 33), (2100, 768, 65), (1030, 2048, 300)])
+def test_captured_and_replayed(kind, rows, cols, m):
+    """Two launches per call, the second under the first; in a graph, with new inputs between replays."""
+    from frink_b200 import device
+    w = device.Weights(fo.encode(kind, synth_weights(2 * rows, cols, 107)), kind, rows, cols, n_mats=2)
+    xs = [torch.from_numpy(synth_acts(m, cols, 108 + i)).cuda() for i in range(3)]
+    off = torch.tensor([0, m // 3, m], dtype=torch.int32, device="cuda")
+    calls = [lambda v, y: device.gemm(w, v, mat=1, out=y), lambda v, y: device.gemm_static(w, v, mat=1, out=y),
+             lambda v, y: device.gemm_grouped(w, off, None, v, m, out=y)]
+    for call in calls:
+        want = [call(v, None).clone() for v in xs]
+        x, y = xs[0].clone(), torch.empty((2, m, rows), device="cuda")
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            call(x, y[0])
+            call(x, y[1])        # the second call's quantizer writes the block that the first call's GEMM reads
+        for v, ref in zip(xs[1:] + xs[:1], want[1:] + want[:1]):
+            x.copy_(v)
+            y.fill_(float("nan"))
+            g.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(y[0], ref) and torch.equal(y[1], ref)
+    assert device.device_error() == 0
