@@ -746,13 +746,13 @@ int launch_by_kind(fk_ctx* ctx, cudaStream_t st, const GemmArgs& a, int kind, co
 //   waves * (runs / split * us_per_run(bn) + (split > 1) * exchange(bn)),   waves = CTAs / (SMs * CTAs per SM)
 //
 // The constants were measured on B200 (us; Q4_K, 3072 x 3072, cold L2; the other kinds are within 20 % below, but MXFP4 in
-// 128-token tiles takes 0.80): a 128-token tile takes 0.68 a run of 32 K, a 64-token one 0.47, a 32-token one 0.42 alone on its SM and 0.56 beside another; the parts
-// of a split tile take 6 to 8 to meet.  A tile's own time falls far less than its width -- its warps walk the same chain per
-// run -- so what a short prompt needs is more CTAs, not only narrower ones: 3072 x 3072, M = 128 was 24 CTAs and 95 us, and
-// is 96 CTAs and 32 us; 3072 x 8192 Q6_K, M = 77 204 -> 77 us; 512 x 3072, M = 16 93 -> 17 us; 8192 x 3072, M = 512 keeps
-// whole 128-token tiles (142 us; 64-token tiles 181, 32-token ones 204).  Grouped: `tiles` expects half a tile of padding
-// per expert, which is what 32-token tiles win by (128 experts, 8 of them for each of 77 rows, 768 x 2048 Q4_K: the routed
-// layer takes 540 us against 755 with 64-token tiles and 1076 with 128).
+// 128-token tiles takes 0.80): a 128-token tile takes 0.68 a run of 32 K, a 64-token one 0.47, a 32-token one 0.42 alone on
+// its SM and 0.56 beside another; the parts of a split tile take 6 to 8 to meet.  A tile's own time falls far less than its
+// width -- its warps walk the same chain per run -- so what a short prompt needs is more CTAs, not only narrower ones
+// (us, whole 128-token tiles in one part against the plan's): 3072 x 3072, M = 128 71 -> 32; 3072 x 8192 Q6_K, M = 77
+// 146 -> 75; 512 x 3072, M = 16 71 -> 17; 8192 x 3072, M = 512 keeps whole 128-token tiles (138; 64-token tiles 177, 32-token
+// ones 200).  Grouped: `tiles` expects half a tile of padding per expert, which is what 32-token tiles win by (128 experts, 8
+// of them for each of 77 rows, 768 x 2048 Q4_K: 169 us against 230 with 64-token tiles and 345 with 128).
 struct GemmPlan { int bn, split; };
 
 GemmPlan gemm_plan(const fk_ctx* ctx, const fk_weight_s* w, int m, bool grouped) {

@@ -1744,7 +1744,7 @@ int launch_kind(fk_ctx* ctx, cudaStream_t st, const GemvArgs& a, const fk_weight
         if (fits) return rc;
     }
     // The block-owned Q4_K kernel takes the plain matvec (and the integer test hook): in a chain of those it is
-    // 4.3 us against 5.4 us a launch (8192 x 3072).  It waits for its whole share before the first dot product, which
+    // 3.8 to 4.0 us against 5.4 us a launch (8192 x 3072).  It waits for its whole share before the first dot product, which
     // costs it inside a decoder step, where the kernel before a matvec is short and hides nothing (688 against 798
     // tokens per second on the 3B Llama shape): the fused and indexed forms keep the general kernel and its rings.
     const bool plain = !a.ids && !a.n_active && !a.norm_w && !a.glu_up && !a.pair_glu && !a.accumulate && !a.ar_on && !a.bias;
